@@ -602,7 +602,7 @@ int inmsom_read_checkpoint(inmsom_ctx *ctx, const char *path, double *ubrtr_e, d
  * every member's RHS at each substep.  group must be even (it keeps each
  * member's state in its set, so the graph can be replayed).  *ms receives
  * the device time of the run.  Creation re-cuts each member's work items
- * to 16 rows at least (a context alone cuts down to 4, which spreads a
+ * to 16 rows at least (a context alone cuts down to 1 or 2, which spreads a
  * small basin over more SMs; in an ensemble the other members fill them),
  * and the members keep that cut after the ensemble is destroyed. */
 typedef struct inmsom_ens inmsom_ens;

@@ -1250,7 +1250,7 @@ int inmsom_ens_create(inmsom_ens **out, inmsom_ctx *const *members, int n, int g
     for (int i = 0; i < n && ce == cudaSuccess; i++) ce = cudaEventCreateWithFlags(&e->join[i], cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaMalloc(&e->d_base, sizeof(int));
     // members share the device: items of 16 rows at least (a basin alone
-    // cuts down to 4 to spread a small basin over more SMs)
+    // cuts down to 1 or 2 to spread a small basin over more SMs)
     for (int i = 0; i < n && ce == cudaSuccess; i++) {
         inmsom_ctx *c = members[i];
         if (c->plan.min_rows == ENS_MIN_ROWS) continue;

@@ -1171,63 +1171,102 @@ std::vector<uint8_t> ocean_rows(const Plan &p, const Dom &d, const float *lu)
     return oc;
 }
 
-// Work items of one variant: each strip's rows rf..rl (device rows; the
-// interior unless a row strip computes into its halo) cut into chunks of
-// about equal cost.  rows_per_item = 0: as many items in all as one wave of
-// resident CTAs holds (`slots`), so that the wave finishes together; else
-// about that many rows per item (several waves).  A row whose written
-// columns are all land skips the momentum stages and costs about LAND_COST
-// of an ocean row; no chunk is shorter than p.min_rows rows (each pays
-// three warm-up iterations: 4 rows for a basin alone, where the items of a
-// small basin would otherwise fill few SMs; 16 for an ensemble member, whose
-// neighbours fill the rest).
+// Work items of one variant over device rows rf..rl (the interior unless a
+// row strip computes into its halo).  A row whose written columns are all
+// land writes nothing, so a strip is first split into segments at its runs
+// of more than GAP_ROWS such rows, which no item covers (a shorter run stays
+// inside its segment: starting an item again costs WARM rows).  On the
+// 2048 x 1536 basin with 40 % land this leaves 66 % of the strips' rows:
+// 66.5 against 78.6 us per substep with every row covered.
+//
+// The segments are then cut into chunks of about equal cost.  rows_per_item
+// = 0: the lowest cost per chunk at which all of them are `waves` waves of
+// the `slots` resident CTAs; else about that many rows per item.  The number
+// of waves is the one that leaves about WAVE_ROWS rows per item, MAX_WAVES
+// at most: CTAs of one wave progress unevenly, and later waves fill the SMs
+// that finish first as long as the items stay long against their warm-up
+// (2048 x 1536: 67.5, 66.5, 67.5, 68.9 us with 1, 2, 3, 4 waves; 4096^2 with
+// FP32 velocities: 373, 335, 327, 322 us).  A land row inside a segment
+// skips the momentum stages and costs about LAND_COST of an ocean row.
+//
+// No chunk is cut shorter than p.min_rows rows (16 for an ensemble member,
+// whose neighbours fill the SMs).  A basin alone goes down to 2 rows, and to
+// 1 where that is at most 3/4 of a wave: such a basin is bound by the latency
+// of an item's chain of rows (us per substep with 4, 2 and 1 rows: 256^2
+// basin, 2286 rows in all: 8.1, 5.4, 6.1; 300 x 200 with land, 1500 rows:
+// 8.5, 6.7, 5.9; 64^2: 8.0, 4.7, 3.8).
+constexpr int GAP_ROWS = 8;     // longest run of land rows inside an item
+constexpr double WARM = 2.5;    // an item's warm-up iterations, in ocean rows
+constexpr int WAVE_ROWS = 10, MAX_WAVES = 8;
+
 std::vector<int4> partition(const Plan &p, const Dom &d, int slots, int rows_per_item, int rf, int rl)
 {
-    const int ny = rl - rf + 1, nya = d.nya();
-    std::vector<std::vector<double>> cost(p.nstrips, std::vector<double>(ny));
-    std::vector<double> total(p.nstrips, 0.0);
-    double all = 0.0;
+    struct Segment {
+        int strip, r0, r1;          // rows r0..r1, the first and last with ocean
+        double cost;
+        int n;
+    };
+    const int nya = d.nya();
+    auto ocean = [&](int s, int r) { return p.ocean[(size_t)s * nya + r] != 0; };
+    std::vector<Segment> seg;
     for (int s = 0; s < p.nstrips; s++) {
-        for (int r = 0; r < ny; r++) {
-            cost[s][r] = p.ocean[(size_t)s * nya + rf + r] ? 1.0 : LAND_COST;
-            total[s] += cost[s][r];
-        }
-        all += total[s];
-    }
-    const int maxc = std::max(1, ny / std::max(1, p.min_rows));
-    std::vector<int> n(p.nstrips);
-    if (rows_per_item > 0) {
-        for (int s = 0; s < p.nstrips; s++)
-            n[s] = std::min(maxc, std::max(1, (ny + rows_per_item / 2) / rows_per_item));
-    } else {
-        // chunks per strip in proportion to its cost (largest remainder)
-        const int want = std::min(std::max(slots, p.nstrips), p.nstrips * maxc);
-        std::vector<std::pair<double, int>> frac;
-        int used = 0;
-        for (int s = 0; s < p.nstrips; s++) {
-            const double exact = all > 0.0 ? want * total[s] / all : 1.0;
-            n[s] = std::min(maxc, std::max(1, (int)exact));
-            used += n[s];
-            frac.push_back({exact - (int)exact, s});
-        }
-        std::sort(frac.begin(), frac.end(), [](const std::pair<double, int> &a, const std::pair<double, int> &b) {
-            return a.first > b.first;
-        });
-        for (size_t t = 0; used < want && t < frac.size(); t++)
-            if (n[frac[t].second] < maxc) n[frac[t].second]++, used++;
-    }
-    // cut each strip at equal shares of its cumulative cost
-    std::vector<int4> items;
-    for (int s = 0; s < p.nstrips; s++) {
-        const double share = total[s] / n[s];
-        double acc = 0.0;
-        int start = rf, made = 0;
+        int land = GAP_ROWS + 1;
         for (int r = rf; r <= rl; r++) {
-            acc += cost[s][r - rf];
-            const bool last_row = r == rl;
-            const bool cut = made < n[s] - 1 && acc >= share * (made + 1) && rl - r >= n[s] - 1 - made;
-            if (cut || last_row) {
-                items.push_back(make_int4(s * p.outw, start, r + 1, 0));
+            if (!ocean(s, r)) {
+                land++;
+                continue;
+            }
+            if (land > GAP_ROWS) seg.push_back({s, r, r, 0.0, 1});
+            else seg.back().cost += land * LAND_COST;
+            seg.back().r1 = r;
+            seg.back().cost += 1.0;
+            land = 0;
+        }
+    }
+    std::vector<int4> items;
+    if (seg.empty()) {              // no ocean: one item that writes nothing
+        items.push_back(make_int4(0, rf, rf + 1, 0));
+        return items;
+    }
+    long long rows = 0;
+    for (const Segment &g : seg) rows += g.r1 - g.r0 + 1;
+    const int min_rows = p.min_rows <= 2 && rows <= slots * 3LL / 4 ? 1 : std::max(1, p.min_rows);
+    auto most = [&](const Segment &g) { return std::max(1, (g.r1 - g.r0 + 1) / min_rows); };
+    if (rows_per_item > 0) {
+        for (Segment &g : seg)
+            g.n = std::min(most(g), std::max(1, (g.r1 - g.r0 + 1 + rows_per_item / 2) / rows_per_item));
+    } else {
+        const long long waves = std::min<long long>(MAX_WAVES, std::max<long long>(1, std::llround((double)rows / slots / WAVE_ROWS)));
+        // chunks per segment at a cost per chunk of at most t (bisection)
+        auto cut = [&](double t) {
+            long long all = 0;
+            for (Segment &g : seg) {
+                g.n = std::min(most(g), std::max(1, (int)std::ceil(g.cost / std::max(t - WARM, 1e-3))));
+                all += g.n;
+            }
+            return all;
+        };
+        double lo = WARM, hi = WARM + 1.0;
+        for (const Segment &g : seg) hi = std::max(hi, WARM + g.cost);
+        for (int k = 0; k < 48; k++) {
+            const double t = 0.5 * (lo + hi);
+            if (cut(t) <= waves * slots) hi = t;
+            else lo = t;
+        }
+        (void)cut(hi);
+    }
+    // cut each segment at equal shares of its cumulative cost
+    for (const Segment &g : seg) {
+        const double share = g.cost / g.n;
+        double acc = 0.0;
+        int start = g.r0, made = 0;
+        for (int r = g.r0; r <= g.r1; r++) {
+            acc += ocean(g.strip, r) ? 1.0 : LAND_COST;
+            // the rows left always suffice for the chunks left: cut at the
+            // latest when there is one row for each
+            const bool cut = made < g.n - 1 && (acc >= share * (made + 1) || g.r1 - r <= g.n - 1 - made);
+            if (cut || r == g.r1) {
+                items.push_back(make_int4(g.strip * p.outw, start, r + 1, 0));
                 start = r + 1;
                 made++;
             }
@@ -1240,11 +1279,6 @@ std::vector<int4> partition(const Plan &p, const Dom &d, int slots, int rows_per
 {
     return partition(p, d, slots, rows_per_item, d.ny_start - d.bnd_y1, d.ny_end - d.bnd_y1);
 }
-
-// waves of work items per table: one for the plain substep (measured on the
-// 2048 x 1536 basin: 2 waves +5.6 %, 1.5 waves +15 %), two for the
-// time-mean substeps (-1.9 % against one)
-int item_waves(int table) { return table == 2 || table == 3 ? 2 : 1; }
 
 // Replaces table v.  On failure the plan keeps its previous table (a
 // launch never sees a count without its items).
@@ -1549,7 +1583,7 @@ int setup(Plan &p, const Dom &d, const Consts &c, const float *const masks[7], c
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     p.nsm = nsm;
     // one item table per variant for the plain substep and one for the
-    // time-mean substeps, each one wave of the kernel's resident CTAs
+    // time-mean substeps, cut for the kernel's resident CTAs
     int occ[NTABLE] = {1, 1, 1, 1, 1};
     cudaError_t oe = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[0], k_substep<false, 3>, NL,
                                                                    ring_bytes<false, 3>());
@@ -1566,7 +1600,7 @@ int setup(Plan &p, const Dom &d, const Consts &c, const float *const masks[7], c
     p.ocean = ocean_rows(p, d, masks[0]);
     for (int v = 0; v < NTABLE; v++) {
         p.occ[v] = occ[v] < 1 ? 1 : occ[v];
-        if (upload_items(p, v, partition(p, d, item_waves(v) * nsm * p.occ[v], 0), s)) return 1;
+        if (upload_items(p, v, partition(p, d, nsm * p.occ[v], 0), s)) return 1;
     }
     p.rows_per_item[0] = p.rows_per_item[1] = 0;
     return 0;
@@ -1745,7 +1779,7 @@ int repartition(Plan &p, const Dom &d, int rows_per_item, cudaStream_t s)
 {
     for (int v = 0; v < NTABLE; v++) {
         p.rows_per_item[v & 1] = rows_per_item;
-        if (upload_items(p, v, partition(p, d, item_waves(v) * p.nsm * p.occ[v], rows_per_item), s)) return 1;
+        if (upload_items(p, v, partition(p, d, p.nsm * p.occ[v], rows_per_item), s)) return 1;
     }
     return 0;
 }
@@ -1806,7 +1840,7 @@ const Plan::ExtTable *ext_table(Plan &p, const Dom &d, int gen, int es, int en, 
         if (t.gen == gen && t.s == es && t.n == en) return &t;
     const int rf = d.ny_start - d.bnd_y1 - es, rl = d.ny_end - d.bnd_y1 + en;
     if (es < 0 || en < 0 || rf < 2 || rl + 2 > d.nya() - 1) return nullptr;
-    const std::vector<int4> items = partition(p, d, item_waves(gen) * p.nsm * p.occ[gen], 0, rf, rl);
+    const std::vector<int4> items = partition(p, d, p.nsm * p.occ[gen], 0, rf, rl);
     Plan::ExtTable t{gen, es, en, (int)items.size(), nullptr};
     if (cudaMalloc(&t.items, items.size() * sizeof(int4)) != cudaSuccess) return nullptr;
     p.ext.push_back(t);   // owned by the plan from here on (freed by release)

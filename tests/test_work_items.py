@@ -1,0 +1,58 @@
+"""Work items of the fused path on basins whose strips hold runs of land:
+items cover the ocean rows of a strip and land runs of up to eight rows
+between them, and are cut down to one row on a small basin.  Against the
+oracle after 10 steps; the fused path's tolerance is 1e-12 normwise."""
+import numpy as np
+import pytest
+from conftest import rel_err
+
+from inmsom_elfs_b200 import basins
+from inmsom_elfs_b200.grid import STATE
+
+
+def _banded(ora, nx, ny, bands, seed):
+    """A beta-plane basin with land across its rows: bands of (first interior
+    row, rows), and one lone ocean row between two of them at the east end."""
+    b = basins.beta_plane_basin(n=nx, ny=ny, seed=seed)
+    j0 = b.bounds.ny_start - b.bounds.bnd_y1
+    for first, rows in bands:
+        b.masks["lu"][: 3 * nx // 4, j0 + first:j0 + first + rows] = 0.0
+        b.masks["lu"][3 * nx // 4:, j0 + first + 1:j0 + first + rows] = 0.0
+    b.hhq_rest[b.masks["lu"] < 0.5] = 0.0
+    basins.finalize(b, ora.OracleBackend())
+    rng = np.random.default_rng(seed)
+    for k in ("ssh_e", "sshp_e"):
+        b.state[k] = np.asfortranarray(0.1 * rng.standard_normal(b.bounds.shape) * b.masks["lu"])
+    ora.hh_init_external(b)
+    return b
+
+
+# land runs shorter than, at and past the eight rows an item spans; sizes
+# from one row per item to several rows, and strips of one or two columns
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,bands", [
+    (31, 40, [(3, 1), (9, 7), (20, 8), (31, 5)]),
+    (62, 60, [(2, 9), (13, 8), (23, 10), (40, 20)]),
+    (400, 170, [(10, 9), (21, 8), (60, 30), (100, 1), (140, 12)]),
+    (700, 500, [(1, 40), (60, 9), (200, 8), (300, 100)]),
+])
+@pytest.mark.parametrize("call", [False, True])
+def test_land_runs_in_the_strips(gpu, ora, nx, ny, bands, call):
+    b = _banded(ora, nx, ny, bands, seed=nx + ny)
+    bo, bg = b.copy(), b.copy()
+    with gpu.BarotropicSolver(bg, resident=True) as s:
+        assert s.path()[0] == 1
+        s.load_state()
+        if call:
+            ora.barotropic_dynamics(bo, 5 * b.dt, 5)
+            s.barotropic_dynamics(5 * b.dt, 5)
+        else:
+            ora.run_substeps(bo, 10, b.dt)
+            s.run_substeps(10, b.dt)
+        s.sync_to_host()
+    for k in STATE:
+        assert rel_err(bg.state[k], bo.state[k]) <= 1e-12, k
+        assert np.array_equal(bg.state[k][b.masks["lu"] < 0.5], b.state[k][b.masks["lu"] < 0.5]), k
+    if call:
+        for k, v in bo.means.items():
+            assert rel_err(bg.means[k], v) <= 1e-12, k
