@@ -24,14 +24,15 @@
 // branch-free (masked selects, predicated stores) except for warp-wide skips
 // of rows without ocean.
 //
-// Input rows j-2..j+1 sit in a ring of RING shared-memory slots.  A slot
+// Input rows j-1..j+1 sit in a ring of RING shared-memory slots.  A slot
 // holds a 36-column segment of the six state fields and of the static
 // fields (rest depth, forcing; in the general variant also viscosity, drag
 // and water flux), brought by two 3-D tiled TMA loads from field-blocked
-// arrays (cp.async.bulk.tensor, each copy for one CTA), plus the row's T-mask bits
-// (and, in the general variant, its metric coefficients) by 1-D bulk copies.
-// One elected lane refills the slot of row j-2 with row j-2+RING once every
-// lane is past it.  Every wait is bounded: on timeout the CTA sets a status bit,
+// arrays (cp.async.bulk.tensor, each copy for one CTA), plus the strip's T-mask bits
+// and Coriolis factor of the row (and, in the general variant, its metric
+// coefficients) by 1-D bulk copies.  One elected lane refills the slot of row
+// j-1 with row j-1+RING once every lane is past it; the few values of it that
+// the next iteration reads are carried in registers.  Every wait is bounded: on timeout the CTA sets a status bit,
 // drains its own copies (bounded) and returns.
 //
 // Two variants: UNI for square uniform grids (every metric array equal to
@@ -64,12 +65,11 @@ struct alignas(64) Params {
     double *dst[NSET];
     float *vdst[4];        // FP32-velocity kernel: u, up, v, vp of the destination
     double *acc[4];
-    const uint32_t *bits;
+    const RowRec *rec;     // per strip and row: T-mask bits and Coriolis factor
     const RowCoef *rows;
-    const double *cor;
-    const int4 *items;     // work items {g0, first row, end row (exclusive), 0}
+    const int4 *items;     // work items {g0, first row, end row (exclusive), strip}
     long long pitch;
-    int bm_words;
+    int nya;               // device rows
     int c_first, c_last;   // interior device columns
     double two_ti, gam, rhs_scale, mu0, rd0, wq0, inv_rho;
     // time means: a substep adds ca * (old level's term) + cb * (new level's)
@@ -153,15 +153,21 @@ struct Layout {
     static constexpr int COEF_OFF = STAT_OFF + NS * SEG * 8;             // general variant: RowCoef
     static constexpr int RHS_OFF = F32 ? (COEF_OFF + 127) / 128 * 128 : COEF_OFF;   // FP32 RHSx, RHSy
     static constexpr int BITS_OFF = F32 ? RHS_OFF + 2 * VSEG * 4 : COEF_OFF + (GEN ? (int)sizeof(RowCoef) : 0);
-    static constexpr int SLOT_B = (BITS_OFF + 32 + 127) / 128 * 128;
+    static constexpr int SLOT_B = (BITS_OFF + (int)sizeof(RowRec) + 127) / 128 * 128;
     static constexpr uint32_t row_tx =
         (uint32_t)((F32 ? 4 * VSEG * 4 + 2 * SEG * 8 + 2 * VSEG * 4 : NSET * SEG * 8) + NS * SEG * 8 +
-                   (GEN ? (int)sizeof(RowCoef) : 0) + 32);
+                   (GEN ? (int)sizeof(RowCoef) : 0) + (int)sizeof(RowRec));
 };
 
-// ring slots: rows j-2..j+1 in use plus one row in flight for the plain
-// substep (16 CTAs per SM fit, 20 with FP32 velocities), two in flight where
-// the registers hold the CTAs per SM to 12 (time-mean sums)
+// ring slots: rows j-1..j+1 in use plus two rows in flight for the plain
+// substep (16 CTAs per SM fit, 20 with FP32 velocities), three in flight
+// where the registers hold the CTAs per SM to 12 (time-mean sums).  What
+// iteration j reads of row j-2 is carried in registers (v at two levels, H
+// + SSH at two levels), which frees its slot an iteration earlier: with one
+// row in flight a quarter of the warps' time went to waiting for rows, the
+// copies' latency being about that of an iteration.  us per substep, before
+// and after: 2048 x 1536 67.3 -> 63.1 (FP32 velocities 55 -> 52), 4096^2
+// FP32 322 -> 309, 256^2 5.4 -> 5.0, 512^2 10.7 -> 9.9
 template <bool GEN, int MODE, bool F32 = false>
 __host__ __device__ constexpr int ring_slots()
 {
@@ -205,7 +211,7 @@ static_assert(Layout<false, true>::BITS_OFF % 16 == 0 && (Layout<false, true>::V
 template <bool GEN, bool F32 = false>
 __device__ __forceinline__ void issue_row(unsigned char *slot, uint64_t *bar, const CUtensorMap *src,
                                           const CUtensorMap *stat, const CUtensorMap *ssh, const CUtensorMap *rhs,
-                                          const void *coef, const void *bits, int x, int row)
+                                          const void *coef, const void *rec, int x, int row)
 {
     using L = Layout<GEN, F32>;
     const int z = 0;
@@ -225,12 +231,12 @@ __device__ __forceinline__ void issue_row(unsigned char *slot, uint64_t *bar, co
             " [%11], [%12, {%9, %5, %6}], [%0];\n\t"
             "@P cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
             " [%15], [%16, {%4, %5, %6}], [%0];\n\t"
-            "@P cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%13], [%14], 32, [%0];\n\t"
+            "@P cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%13], [%14], 16, [%0];\n\t"
             "}" ::"r"(smem_addr(bar)),
             "r"(L::row_tx), "r"(smem_addr(slot)), "l"(reinterpret_cast<uint64_t>(src)), "r"(x4), "r"(row), "r"(z),
             "r"(smem_addr(slot + L::SSH_OFF)), "l"(reinterpret_cast<uint64_t>(ssh)), "r"(x), "r"(zs),
             "r"(smem_addr(slot + L::STAT_OFF)), "l"(reinterpret_cast<uint64_t>(stat)),
-            "r"(smem_addr(slot + L::BITS_OFF)), "l"(bits),
+            "r"(smem_addr(slot + L::BITS_OFF)), "l"(rec),
             "r"(smem_addr(slot + L::RHS_OFF)), "l"(reinterpret_cast<uint64_t>(rhs))
             : "memory");
     } else if constexpr (GEN) {
@@ -243,12 +249,12 @@ __device__ __forceinline__ void issue_row(unsigned char *slot, uint64_t *bar, co
             "@P cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
             " [%7], [%8, {%4, %5, %6}], [%0];\n\t"
             "@P cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%9], [%10], %11, [%0];\n\t"
-            "@P cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%12], [%13], 32, [%0];\n\t"
+            "@P cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%12], [%13], 16, [%0];\n\t"
             "}" ::"r"(smem_addr(bar)),
             "r"(L::row_tx), "r"(smem_addr(slot)), "l"(reinterpret_cast<uint64_t>(src)), "r"(x), "r"(row), "r"(z),
             "r"(smem_addr(slot + L::STAT_OFF)), "l"(reinterpret_cast<uint64_t>(stat)),
             "r"(smem_addr(slot + L::COEF_OFF)), "l"(coef), "n"((int)sizeof(RowCoef)),
-            "r"(smem_addr(slot + L::BITS_OFF)), "l"(bits)
+            "r"(smem_addr(slot + L::BITS_OFF)), "l"(rec)
             : "memory");
     } else {
         (void)coef;
@@ -261,11 +267,11 @@ __device__ __forceinline__ void issue_row(unsigned char *slot, uint64_t *bar, co
             " [%2], [%3, {%4, %5, %6}], [%0];\n\t"
             "@P cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
             " [%7], [%8, {%4, %5, %6}], [%0];\n\t"
-            "@P cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%9], [%10], 32, [%0];\n\t"
+            "@P cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%9], [%10], 16, [%0];\n\t"
             "}" ::"r"(smem_addr(bar)),
             "r"(L::row_tx), "r"(smem_addr(slot)), "l"(reinterpret_cast<uint64_t>(src)), "r"(x), "r"(row), "r"(z),
             "r"(smem_addr(slot + L::STAT_OFF)), "l"(reinterpret_cast<uint64_t>(stat)),
-            "r"(smem_addr(slot + L::BITS_OFF)), "l"(bits)
+            "r"(smem_addr(slot + L::BITS_OFF)), "l"(rec)
             : "memory");
     }
 }
@@ -358,14 +364,15 @@ struct S1 {
     R U, Ul, V, Vr;          // U = u*hu at k, k-1; V = v*hv at k, k+1
     R Ru;                    // u equation of row j: forcing + pressure gradient - drag
     R Rv;                    // v equation of row j: forcing + pressure gradient - drag
-    R cor;                   // uniform variant: Coriolis factor of row j
     R slx, sly;              // pressure-gradient terms (time means only)
     HQ<R> hq;                // H + ssh of row j+1
 };
 // values of row j-1 from stage 2 (and of stage 1 routed on), carried on
 template <class R>
 struct S2 {
-    double sn;               // new SSH of the row
+    double sn;               // new SSH of the row (time means only)
+    double hs, hsn;          // H + previous SSH and H + new SSH of the row
+    R vm, vpm;               // v, vp of the row
     R V, Uo;                 // V and U of the row
     R vs;                    // v(k) + v(k+1) of the row
     R Cu;                    // the row's part of the u equation of the row above
@@ -401,8 +408,7 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
     const int k = g0 + 2 + l;                  // this lane's column
     const int r0 = item.y, r1 = item.z;        // output rows [r0, r1), r1 > r0
     const int row_lo = r0 - 2, row_hi = r1 + 1;             // rows kept in the ring
-    const int wbase = (g0 >> 7) << 2;                       // first mask word of the window
-    const int bsh = k - wbase * 32;                         // bit of k in the window
+    const RowRec *const rec = p.rec + (size_t)item.w * p.nya;   // this strip's records, by device row
     const unsigned char *lane = ring + (l + 2) * 8;         // this lane's column in a segment
     const unsigned char *lane32 = ring + (l + 2 + (g0 & 3)) * 4;   // ... in an FP32 segment (from g0 & ~3)
 
@@ -415,11 +421,11 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
     auto issue = [&](int row, int slot) {
         if ((int)blockIdx.x == p.hold_item && row == min(row_lo + p.hold_row, row_hi)) return;   // test hook
         issue_row<GEN, F32>(ring + slot * L::SLOT_B, &mbar[slot], tm_src, &p.tm_stat, &p.tm_ssh, &p.tm_rhs, p.rows + row,
-                       p.bits + (size_t)row * p.bm_words + wbase, g0, row);
+                       rec + row, g0, row);
     };
     auto mask2 = [&](int o) -> uint32_t {   // bits: lu(k), lu(k+1)
-        const uint32_t *w = reinterpret_cast<const uint32_t *>(ring + o + L::BITS_OFF);
-        return __funnelshift_r(w[bsh >> 5], w[(bsh >> 5) + 1], bsh & 31) & 3u;
+        const uint2 w = *reinterpret_cast<const uint2 *>(ring + o + L::BITS_OFF);
+        return __funnelshift_r(w.x, w.y, l) & 3u;
     };
 
     if (l == 0) {
@@ -440,8 +446,8 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
                 f_rd0 = (float)p.rd0, f_mu0 = (float)p.mu0;
 #define RK(pv, fv) pick_real<F32>((pv), (fv))
 
-    // slots of rows j-2, j-1, j, j+1 and the fill parity of row j+1
-    int i_m2 = RING - 1, i_m1 = 0, i_0 = 1, i_p1 = 2;
+    // slots of rows j-1, j, j+1 and the fill parity of row j+1
+    int i_m1 = 0, i_0 = 1, i_p1 = 2;
     uint32_t ph = 0;
     // T-mask bits, 2 per row: row j+1 in bits 0-1, j in 2-3, j-1 in 4-5, j-2 in 6-7
     uint32_t mk = 0;
@@ -468,7 +474,7 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
         constexpr bool D1 = decltype(on1)::value, D2 = decltype(on2)::value;
         constexpr bool D3U = decltype(on3u)::value, D3V = decltype(on3v)::value;
         if (!ok) return;
-        const int o_m2 = i_m2 * L::SLOT_B, o_m1 = i_m1 * L::SLOT_B, o_0 = i_0 * L::SLOT_B, o_p1 = i_p1 * L::SLOT_B;
+        const int o_m1 = i_m1 * L::SLOT_B, o_0 = i_0 * L::SLOT_B, o_p1 = i_p1 * L::SLOT_B;
         if constexpr (D1) {   // stage 1 reads row j+1
             if (!__all_sync(0xffffffffu, ready)) {
                 ok = __all_sync(0xffffffffu, mbar_wait(&mbar[i_p1], ph, p.wait_limit));
@@ -527,7 +533,6 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
                 sly = -(R)(e1v - e0) * RK(p.gd, f_gd) * hv;
                 rdu = rdv = RK(p.rd0, f_rd0);
                 au = av = RK(p.d2, f_d2);
-                n.cor = (R)p.cor[j];
             }
             // RHS: from the ring (FP64 state) or from the FP32 copy
             const R rx = F32 ? (R)*reinterpret_cast<const float *>(lane32 + o_0 + L::RHS_OFF) : (R)AT(o_0, T_RX, 0);
@@ -545,15 +550,18 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
 
         // ---------------- stage 2: row rho = j-1 -------------------------
         double sn;
+        double hsn;
         R FX, FY, GY, ST, SS, QU, QV, vs, u_r, up_r, v_m, vp_m;
+        const double h0 = AT(o_m1, T_H, 0);
+        const double hs = h0 + AS(o_m1, S_SSHP, 0);   // H + previous SSH of row j-1
         if constexpr (D2) {
             const uint32_t mr = (mk >> 4) & 3u, mu_ = (mk >> 2) & 3u;   // rows rho, rho+1
             const int lc = mr & 1, lr = (mr >> 1) & 1, lu = mu_ & 1, lur = (mu_ >> 1) & 1;
             const int luu = lc & lr & lu & lur;
             u_r = AV(o_m1, S_U, 0);
             up_r = AV(o_m1, S_UP, 0);
-            v_m = AV(o_m2, S_V, 0);
-            vp_m = AV(o_m2, S_VP, 0);
+            v_m = qc.vm;      // row j-2
+            vp_m = qc.vpm;
             const R u_l = AV(o_m1, S_U, -1), u_u = AV(o_0, S_U, 0);
             const R v_r = AV(o_m1, S_V, 0), v_rr = AV(o_m1, S_V, 1);
             const R up_l = AV(o_m1, S_UP, -1), up_u = AV(o_0, S_UP, 0);
@@ -570,6 +578,7 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
             const double div = GEN ? (c.U - c.Ul) * CF(o_m1, c_u) + c.V * CF(o_m1, c_v0) - qc.V * CF(o_m1, c_v1)
                                    : (((double)c.U - (double)c.Ul) + ((double)c.V - (double)qc.V)) * p.inv_d;
             sn = sel(lc, AS(o_m1, S_SSHP, 0) + two_ti * (wq - div));
+            hsn = h0 + sn;
             // vel_ssh.f90:63-73, :88-98 advective fluxes on T and h faces
             vs = v_r + v_rr;
             FX = (c.Ul + c.U) * (u_l + u_r) * (GEN ? (R)CF(o_m1, fx) : RK(p.d4, f_d4));
@@ -586,7 +595,7 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
                 if (!p.vort_zero)
                     cor += sel(luu, (v_rr - v_r) * CF(o_m1, vt0) - u_u * CF(o_m1, vt1) + u_r * CF(o_m1, vt2));
             } else {
-                cor = c.cor;
+                cor = (R)reinterpret_cast<const RowRec *>(ring + o_m1 + L::BITS_OFF)->cor;
             }
             const R Wh = hh * cor;
             QU = Wh * vs;
@@ -600,11 +609,12 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
             SS = mu_h * hh * str_s;
         }
         R FXr, STr, QVl, SSl;
-        double SNr;
+        double SNr, HSNr;
         if constexpr (D2) {
             FXr = SHFL_DN(FX);
             STr = SHFL_DN(ST);
-            SNr = SHFL_DN(sn);
+            HSNr = SHFL_DN(hsn);
+            if (ACC) SNr = SHFL_DN(sn);
             QVl = SHFL_UP(QV);
             SSl = SHFL_UP(SS);
         }
@@ -627,11 +637,11 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
                 const bool wu = out && (lc & lr), wt = out && lc;
                 const double e0 = AS(o_m1, S_SSH, 0);
                 const double sp0 = AS(o_m1, S_SSHP, 0), sp1 = AS(o_m1, S_SSHP, 1);
-                const double h0 = AT(o_m1, T_H, 0), h1 = AT(o_m1, T_H, 1);
+                const double h1 = AT(o_m1, T_H, 1);
                 // vel_ssh.f90:536-551
                 const R ku2 = GEN ? (R)CF(o_m1, ku2) : R(0.5);
-                const R hup = (R)((h0 + sp0) + (h1 + sp1)) * ku2;
-                const R hun = (R)((h0 + sn) + (h1 + SNr)) * ku2;
+                const R hup = (R)(hs + (h1 + sp1)) * ku2;
+                const R hun = (R)(hsn + HSNr) * ku2;
                 const R difx = GEN ? (R)((STr - ST) * CF(o_m1, dux) + SS * CF(o_m1, dus0)) : ((STr - ST) + SS) * RK(p.d, f_d);
                 const R grx = c.Ru + qc.Cu - ((FXr - FX) + FY) + difx + QU * R(0.25);
                 const R un = (up_r * hup + grx * (GEN ? (R)(two_ti * CF(o_m1, rau)) : RK(p.tt, f_tt))) * rcp_nr(hun);
@@ -658,29 +668,26 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
         if constexpr (D3V) {
             // vel_ssh.f90:88-98 the x flux of v on the h point of row R,
             // from the transports of rows R and R+1
-            const R GX = (GEN ? (R)(qc.Uo * CF(o_m2, gx0) + c.U * CF(o_m2, gx1)) : (qc.Uo + c.U) * RK(p.d4, f_d4)) * qc.vs;
+            const R GX = (GEN ? (R)(qc.Uo * CF(o_m1, pgx0) + c.U * CF(o_m1, pgx1)) : (qc.Uo + c.U) * RK(p.d4, f_d4)) * qc.vs;
             const R GXl = SHFL_UP(GX);
             const uint32_t mR = (mk >> 6) & 3u, mU = (mk >> 4) & 3u;   // rows R, R+1
             if (__any_sync(0xffffffffu, out && (mR & mU & 1u))) {
                 const bool wv = out && (mR & mU & 1u);
-                const double sp0 = AS(o_m2, S_SSHP, 0), sp1 = AS(o_m1, S_SSHP, 0);
-                const double h0 = AT(o_m2, T_H, 0), h1 = AT(o_m1, T_H, 0);
                 const R v0 = v_m, vp0 = vp_m;
-                const double sn0 = qc.sn, sn1 = sn;
                 // vel_ssh.f90:554-569
                 R hvp, hvn;
                 if constexpr (GEN) {
-                    hvp = ((h0 + sp0) * CF(o_m2, wv0) + (h1 + sp1) * CF(o_m2, wv1)) * 0.5;
-                    hvn = ((h0 + sn0) * CF(o_m2, wv0) + (h1 + sn1) * CF(o_m2, wv1)) * 0.5;
+                    hvp = (qc.hs * CF(o_m1, pwv0) + hs * CF(o_m1, pwv1)) * 0.5;
+                    hvn = (qc.hsn * CF(o_m1, pwv0) + hsn * CF(o_m1, pwv1)) * 0.5;
                 } else {
-                    hvp = (R)((h0 + sp0) + (h1 + sp1)) * R(0.5);
-                    hvn = (R)((h0 + sn0) + (h1 + sn1)) * R(0.5);
+                    hvp = (R)(qc.hs + hs) * R(0.5);
+                    hvn = (R)(qc.hsn + hsn) * R(0.5);
                 }
-                const R gry = qc.Pv - (GX - GXl) - GY - ST * (GEN ? (R)CF(o_m2, dvt1) : RK(p.d, f_d));
-                const R vn = (vp0 * hvp + gry * (GEN ? (R)(two_ti * CF(o_m2, rav)) : RK(p.tt, f_tt))) * rcp_nr(hvn);
+                const R gry = qc.Pv - (GX - GXl) - GY - ST * (GEN ? (R)CF(o_m1, pdvt1) : RK(p.d, f_d));
+                const R vn = (vp0 * hvp + gry * (GEN ? (R)(two_ti * CF(o_m1, prav)) : RK(p.tt, f_tt))) * rcp_nr(hvn);
                 const long long idx = gi - 2 * p.pitch;
                 if (ACC && wv) {
-                    const double slyn = -(sn1 - sn0) * (GEN ? CF(o_m2, gdxh) : p.gd) * hvn;
+                    const double slyn = -(sn - qc.sn) * (GEN ? CF(o_m1, pgdxh) : p.gd) * hvn;
                     double a = qc.V * p.ca + vn * hvn * p.cb, b = qc.sly * p.ca + slyn * p.cb;
                     if (ACC == 2) { a += qc.av1; b += qc.av3; }
                     p.acc[1][idx] = a;
@@ -703,22 +710,26 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
             // -ST(rho+1)*dx(rho+1)^2/dxh(rho)
             const R dify = GEN ? (R)(ST * CF(o_m1, dvt0) + (SS - SSl) * CF(o_m1, dvs)) : (ST + (SS - SSl)) * RK(p.d, f_d);
             q.Pv = c.Rv + GY + dify - (QV + QVl) * R(0.25);
-            q.sn = sn;
+            if (ACC) q.sn = sn;
+            q.hsn = hsn;
             q.vs = vs;
         }
+        q.hs = hs;
+        q.vm = AV(o_m1, S_V, 0);
+        q.vpm = AV(o_m1, S_VP, 0);
         q.V = c.V;
         q.Uo = c.U;
         q.hqm = c.hq;
         if (ACC) q.sly = c.sly;
 
-        // row j-2 was last read above: once every lane is past it, its slot
-        // takes row j-2+RING
+        // row j-1 was last read above (what the next iteration needs of it
+        // is carried in registers): once every lane is past it, its slot
+        // takes row j-1+RING
         __syncwarp();
-        if (j - 2 >= row_lo && j - 2 + RING <= row_hi) {
-            issue(j - 2 + RING, i_m2);
-            issued = j - 2 + RING;
+        if (j - 1 + RING <= row_hi) {
+            issue(j - 1 + RING, i_m1);
+            issued = j - 1 + RING;
         }
-        i_m2 = i_m1;
         i_m1 = i_0;
         i_0 = i_p1;
         i_p1 = i_p1 == RING - 1 ? 0 : i_p1 + 1;
@@ -1004,11 +1015,10 @@ Params base_params(const Plan &p, const Dom &d, const Consts &c, const Forcing &
     Params q;
     std::memset(&q, 0, sizeof q);
     q.tm_stat = p.tm_stat[gen];
-    q.bits = p.bits;
+    q.rec = p.rec;
     q.rows = p.rows;
-    q.cor = p.cor;
     q.pitch = d.pitch;
-    q.bm_words = p.bm_words;
+    q.nya = d.nya();
     q.c_first = d.nx_start - d.bnd_x1 + d.xoff;
     q.c_last = d.nx_end - d.bnd_x1 + d.xoff;
     q.mu0 = f.mu0;
@@ -1266,7 +1276,7 @@ std::vector<int4> partition(const Plan &p, const Dom &d, int slots, int rows_per
             // latest when there is one row for each
             const bool cut = made < g.n - 1 && (acc >= share * (made + 1) || g.r1 - r <= g.n - 1 - made);
             if (cut || r == g.r1) {
-                items.push_back(make_int4(g.strip * p.outw, start, r + 1, 0));
+                items.push_back(make_int4(g.strip * p.outw, start, r + 1, g.strip));
                 start = r + 1;
                 made++;
             }
@@ -1302,8 +1312,7 @@ int upload_items(Plan &p, int v, const std::vector<int4> &items, cudaStream_t s)
 void release(Plan &p)
 {
     cudaFree(p.rows);
-    cudaFree(p.cor);
-    cudaFree(p.bits);
+    cudaFree(p.rec);
     // the plan owns the two sets that are not the caller's current state
     cudaFree(p.buf[0][0]);
     cudaFree(p.buf[1][0]);
@@ -1323,8 +1332,7 @@ void release(Plan &p)
     cudaFree(p.stat32);
     p.stat32 = nullptr;
     p.rows = nullptr;
-    p.cor = nullptr;
-    p.bits = nullptr;
+    p.rec = nullptr;
     for (auto &b : p.buf)
         for (auto &x : b) x = nullptr;
     p.stat = nullptr;
@@ -1516,6 +1524,16 @@ int setup(Plan &p, const Dom &d, const Consts &c, const float *const masks[7], c
         q.av = g(DYT, 0) * g(DXH, 0);
         q.rau = 1.0 / q.au;
         q.rav = 1.0 / q.av;
+        // what the v equation of the row above (n-1) reads while row n is
+        // in the ring
+        const RowCoef &o = rows[r > 0 ? r - 1 : 0];
+        q.pgx0 = o.gx0;
+        q.pgx1 = o.gx1;
+        q.pwv0 = o.wv0;
+        q.pwv1 = o.wv1;
+        q.pdvt1 = o.dvt1;
+        q.prav = o.rav;
+        q.pgdxh = o.gdxh;
     }
     p.vort_zero = vz;
     // square uniform grid: every metric array equal to one spacing over the
@@ -1525,28 +1543,27 @@ int setup(Plan &p, const Dom &d, const Consts &c, const float *const masks[7], c
     for (int k = 0; k < 8 && p.uni; k++)
         for (int n = d.bnd_y1 + 1; n <= d.bnd_y2 - 1 && p.uni; n++)
             if (row_of(k, n) != p.d) p.uni = false;
-    std::vector<double> cor(nya);
-    for (int r = 0; r < nya; r++) cor[r] = row_of(RLH, r + d.bnd_y1) * p.d * p.d;
-    // 1-bit T mask indexed by device column, rows padded so that every CTA
-    // window (8 words from a 4-word boundary) lies inside the row
-    p.bm_words = (int)(((d.pitch + 31) / 32 + 8 + 3) / 4 * 4);
-    std::vector<uint32_t> bits((size_t)p.bm_words * nya, 0u);
+    // per strip and row: bit l is the T mask of lane l's column g0+2+l (33
+    // bits in use: lane 31 reads its right neighbour's), and the uniform
+    // variant's Coriolis factor
+    std::vector<RowRec> rec((size_t)p.nstrips * nya);
     const float *lu = masks[0];
-    for (int r = 0; r < nya; r++)
-        for (int col = 0; col < nxa; col++)
-            if (lu[(size_t)r * nxa + col] > 0.5f) {
-                const int dc = col + d.xoff;
-                bits[(size_t)r * p.bm_words + dc / 32] |= 1u << (dc % 32);
+    for (int t = 0; t < p.nstrips; t++)
+        for (int r = 0; r < nya; r++) {
+            RowRec &q = rec[(size_t)t * nya + r];
+            q = RowRec{};
+            for (int l = 0; l <= NL; l++) {
+                const int col = t * p.outw + 2 + l - d.xoff;
+                if (col < nxa && lu[(size_t)r * nxa + col] > 0.5f) (l < 32 ? q.lo : q.hi) |= 1u << (l & 31);
             }
+            q.cor = row_of(RLH, r + d.bnd_y1) * p.d * p.d;
+        }
 
     if (cudaMalloc(&p.rows, rows.size() * sizeof(RowCoef)) != cudaSuccess) return 1;
     if (cudaMemcpyAsync(p.rows, rows.data(), rows.size() * sizeof(RowCoef), cudaMemcpyHostToDevice, s) != cudaSuccess)
         return 1;
-    if (cudaMalloc(&p.cor, cor.size() * sizeof(double)) != cudaSuccess) return 1;
-    if (cudaMemcpyAsync(p.cor, cor.data(), cor.size() * sizeof(double), cudaMemcpyHostToDevice, s) != cudaSuccess)
-        return 1;
-    if (cudaMalloc(&p.bits, bits.size() * sizeof(uint32_t)) != cudaSuccess) return 1;
-    if (cudaMemcpyAsync(p.bits, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, s) != cudaSuccess)
+    if (cudaMalloc(&p.rec, rec.size() * sizeof(RowRec)) != cudaSuccess) return 1;
+    if (cudaMemcpyAsync(p.rec, rec.data(), rec.size() * sizeof(RowRec), cudaMemcpyHostToDevice, s) != cudaSuccess)
         return 1;
     // field-blocked sets: the caller's state block and two ping-pong sets
     p.fstride = d.pitch * nya;

@@ -49,7 +49,16 @@ enum { S_U, S_UP, S_V, S_VP, S_SSH, S_SSHP, NSET };
 // holds all six)
 enum { T_H, T_RX, T_RY, T_MU, T_RD, T_WF, NSTAT };
 
-// per-row coefficients, row index = device row (n - bnd_y1); 38 doubles so
+// per strip and device row, copied with the row: T-mask bits of the strip's
+// columns (bit l: lane l's column) and the uniform variant's Coriolis
+// factor rlh_s*d*d
+struct RowRec {
+    uint32_t lo, hi;
+    double cor;
+};
+static_assert(sizeof(RowRec) == 16, "one 16-byte bulk copy per row");
+
+// per-row coefficients, row index = device row (n - bnd_y1); 44 doubles so
 // that a row is a whole number of 16-byte units for the bulk copies
 struct RowCoef {
     double ku, ku2;           // hu: area(n)/(dxt*dyh)(n), and half of it
@@ -68,7 +77,8 @@ struct RowCoef {
     double gdyh, gdxh;        // g*dyh, g*dxh
     double au, av;            // dxt*dyh, dyt*dxh
     double rau, rav;          // 1/(dxt*dyh), 1/(dyt*dxh)
-    double pad;
+    // of the row above (n-1): gx0, gx1, wv0, wv1, dvt1, rav, gdxh
+    double pgx0, pgx1, pwv0, pwv1, pdvt1, prav, pgdxh;
 };
 static_assert(sizeof(RowCoef) % 16 == 0, "RowCoef must be a multiple of 16 bytes");
 
@@ -80,15 +90,13 @@ struct Plan {
     // time-mean substeps, and the FP32-velocity substep (their kernels hold
     // different numbers of CTAs per SM)
     int nitems[5] = {0, 0, 0, 0, 0};
-    int4 *items[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // {g0, first row, end row, 0} per item
+    int4 *items[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // {g0, first row, end row, strip} per item
     bool uni = false;         // metrics all equal one spacing d (square uniform grid)
     double d = 0.0;           // that spacing
     long long min_pitch = 0;  // device row pitch the strips need
     // device data
     RowCoef *rows = nullptr;        // per-row coefficients (general variant)
-    double *cor = nullptr;          // per-row rlh_s*d*d (uniform variant)
-    uint32_t *bits = nullptr;       // 1-bit T mask, bm_words per row
-    int bm_words = 0;
+    RowRec *rec = nullptr;          // per strip and row: T-mask bits, Coriolis factor
     double *buf[2][6] = {};         // the two ping-pong sets (field views)
     double *set[3] = {};            // base of each state set (field 0)
     double *stat = nullptr;         // static block, NSTAT fields
