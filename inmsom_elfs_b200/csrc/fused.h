@@ -91,6 +91,7 @@ struct Plan {
     // different numbers of CTAs per SM)
     int nitems[5] = {0, 0, 0, 0, 0};
     int4 *items[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // {g0, first row, end row, strip} per item
+    bool turn[5] = {};        // alternate substeps take a table's items from its end
     bool uni = false;         // metrics all equal one spacing d (square uniform grid)
     double d = 0.0;           // that spacing
     long long min_pitch = 0;  // device row pitch the strips need
