@@ -44,7 +44,7 @@ extern "C" {
                                      vbrtr_i, ssh4gradx, ssh4grady).  Without it
                                      every call copies every array argument in
                                      and out. */
-#define INMSOM_FORCE_GENERAL 0x2u /* always use the per-loop kernels (exact
+#define INMSOM_FORCE_GENERAL 0x2u /* always use the general-path kernels (exact
                                      reference rounding) even when the fused
                                      streaming kernel is eligible               */
 #define INMSOM_GUARD         0x4u /* after every call apply the range/NaN guard of
@@ -407,7 +407,7 @@ int inmsom_load_state(inmsom_ctx *ctx, double *ubrtr_e, double *ubrtrp_e,
                       const double *wflux, const double *mu, const double *mu4,
                       const double *rdis);
 
-/* Which kernel path the context uses: 0 = per-loop kernels (exact
+/* Which kernel path the context uses: 0 = general-path kernels (exact
  * reference rounding), 1 = fused streaming kernel.  *reason receives a
  * static string saying why the fused path is not eligible (or "eligible"). */
 int inmsom_gpu_path(inmsom_ctx *ctx, int *path, const char **reason);

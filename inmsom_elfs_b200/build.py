@@ -2,7 +2,7 @@
 
 The library is built in-tree, next to this file, so that it travels with
 the repository.  general.cu and column.cu are compiled with --fmad=false
-(per-loop and per-column kernels that round exactly like the Fortran
+(general-path and per-column kernels that round exactly like the Fortran
 expressions); the fused streaming
 kernel and the C ABI layer use the default contraction.
 """

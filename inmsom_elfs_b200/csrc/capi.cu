@@ -1,6 +1,6 @@
 // C ABI of the barotropic step (include/inmsom_gpu.h): context, device
 // mirrors of the Fortran arrays, host<->device residency, and the drivers
-// that sequence the kernels of general.cu (per-loop, exact rounding) and
+// that sequence the kernels of general.cu (general path, exact rounding) and
 // fused.cu (streaming, one kernel per substep).
 #include "inmsom_gpu.h"
 
@@ -112,48 +112,32 @@ int alloc_set(inmsom_ctx *c, double **arr, int n)
 // external depths := hh_init(ssh_e, sshp_e), Function/depth.f90:2-105
 void depths_from_state(inmsom_ctx *c)
 {
-    double **h = c->depth;
-    general::hh_init(c->dom, c->gdev(), c->c, h[H_Q], h[H_QP], h[H_QN], h[H_U], h[H_UP], h[H_UN],
-                     h[H_V], h[H_VP], h[H_VN], h[H_H], h[H_HP], h[H_HN], c->state[S_SSH],
-                     c->state[S_SSHP], c->stream);
+    general::hh_init(c->dom, c->gdev(), c->c, c->depth, c->state[S_SSH], c->state[S_SSHP], c->stream);
     c->depths_current = true;
 }
 
-// One substep of the Function/vel_ssh.f90:484-650 loop body on the work
-// arrays, general path.  acc receives the time-mean sums (may be scratch).
-void general_substep(inmsom_ctx *c, double ti, int nstep, int ksw4, double rhs_scale,
-                     bool shift_depths)
+// The arguments of the general path's substep on the work arrays w
+general::StepArgs step_args(inmsom_ctx *c, double *const w[NWORK], double ti, int nstep)
 {
-    const Dom &d = c->dom;
-    const GridDev g = c->gdev();
-    cudaStream_t s = c->stream;
-    double **w = c->work, **h = c->depth, **f = c->forc, **x = c->scr;
-
-    general::continuity(d, g, c->c, ti, w[W_SSHN], w[W_SSHP], w[W_U], w[W_V], h[H_U], h[H_V],
-                        f[F_WFLUX], s);
-    general::halo(d, w[W_SSHN], s);
-    if (c->c.ffs > 0) general::hh_update(d, g, h[H_QN], h[H_UN], h[H_VN], h[H_HN], w[W_SSHN], s);
-    general::stress_components(d, g, w[W_UP], w[W_VP], x[C_STRT], x[C_STRS], s);
-    general::uv_trans(d, g, w[W_U], w[W_V], x[C_VORT], h[H_U], h[H_V], h[H_H], x[C_ADVX],
-                      x[C_ADVY], s);
-    general::uv_diff2(d, g, f[F_MU], x[C_STRT], x[C_STRS], h[H_Q], h[H_H], x[C_DIFX], x[C_DIFY], s);
-    if (ksw4 > 0)
-        general::uv_diff4(d, g, f[F_MU4], x[C_STRT], x[C_STRS], x[C_FX], x[C_FY], h[H_Q], h[H_U],
-                          h[H_V], h[H_H], x[C_DIFX], x[C_DIFY], s);
-    general::MomentumArgs a;
-    a.un = w[W_UN]; a.vn = w[W_VN];
-    a.ubrtr_i = c->acc[A_UI]; a.vbrtr_i = c->acc[A_VI]; a.gx = c->acc[A_GX]; a.gy = c->acc[A_GY];
-    a.u = w[W_U]; a.v = w[W_V]; a.up = w[W_UP]; a.vp = w[W_VP]; a.ssh = w[W_SSH]; a.sshn = w[W_SSHN];
-    a.hu = h[H_U]; a.hup = h[H_UP]; a.hun = h[H_UN]; a.hv = h[H_V]; a.hvp = h[H_VP]; a.hvn = h[H_VN];
-    a.hh = h[H_H];
-    a.rhsx = f[F_RHSX]; a.rhsy = f[F_RHSY]; a.difx = x[C_DIFX]; a.dify = x[C_DIFY];
-    a.advx = x[C_ADVX]; a.advy = x[C_ADVY]; a.rdis = f[F_RDIS]; a.rhs_scale = rhs_scale;
-    general::momentum(d, g, c->c, ti, nstep, a, s);
-    general::halo(d, w[W_UN], s);
-    general::halo(d, w[W_VN], s);
-    general::asselin3(d, g, c->c, (double)nstep, w[W_SSH], w[W_SSHP], w[W_SSHN], w[W_U], w[W_UP],
-                      w[W_UN], w[W_V], w[W_VP], w[W_VN], s);
-    if (c->c.ffs > 0 && shift_depths) general::hh_shift(d, g, c->c, h, nstep, s);
+    double **h = c->depth, **f = c->forc, **x = c->scr;
+    general::StepArgs a = {};
+    a.u = w[W_U]; a.up = w[W_UP]; a.un = w[W_UN];
+    a.v = w[W_V]; a.vp = w[W_VP]; a.vn = w[W_VN];
+    a.ssh = w[W_SSH]; a.sshp = w[W_SSHP]; a.sshn = w[W_SSHN];
+    a.hq = h[H_Q]; a.hqp = h[H_QP]; a.hqn = h[H_QN];
+    a.hu = h[H_U]; a.hup = h[H_UP]; a.hun = h[H_UN];
+    a.hv = h[H_V]; a.hvp = h[H_VP]; a.hvn = h[H_VN];
+    a.hh = h[H_H]; a.hhp = h[H_HP]; a.hhn = h[H_HN];
+    a.vort = x[C_VORT]; a.strt = x[C_STRT]; a.strs = x[C_STRS]; a.fx = x[C_FX]; a.fy = x[C_FY];
+    a.advx = x[C_ADVX]; a.advy = x[C_ADVY]; a.difx = x[C_DIFX]; a.dify = x[C_DIFY];
+    a.ui = c->acc[A_UI]; a.vi = c->acc[A_VI]; a.gx = c->acc[A_GX]; a.gy = c->acc[A_GY];
+    a.rhsx = f[F_RHSX]; a.rhsy = f[F_RHSY]; a.wflux = f[F_WFLUX];
+    a.mu = f[F_MU]; a.mu4 = f[F_MU4]; a.rdis = f[F_RDIS];
+    a.rhs_scale = 1.0;
+    a.ti = ti;
+    a.ns = (double)nstep;
+    a.four_nstep = (double)(4 * nstep);
+    return a;
 }
 
 // Function/vel_ssh.f90:465-675 on the device, general path
@@ -161,32 +145,62 @@ void general_dynamics(inmsom_ctx *c, double tau, int nstep, int ksw4)
 {
     const Dom &d = c->dom;
     cudaStream_t s = c->stream;
-    double **w = c->work, **st = c->state;
-    const double ti = tau / (double)nstep;
-    general::fill(d, w[W_UN], 0.0, s);
-    general::fill(d, w[W_VN], 0.0, s);
-    general::fill(d, w[W_SSHN], 0.0, s);
-    general::copy(d, w[W_UP], st[S_UP], s);
-    general::copy(d, w[W_VP], st[S_VP], s);
-    general::copy(d, w[W_SSHP], st[S_SSHP], s);
-    general::copy(d, w[W_U], st[S_U], s);
-    general::copy(d, w[W_V], st[S_V], s);
-    general::copy(d, w[W_SSH], st[S_SSH], s);
-    for (int k = 0; k < NACC; k++) general::fill(d, c->acc[k], 0.0, s);
-    for (int step = 1; step <= 2 * nstep; step++) {
-        general_substep(c, ti, nstep, ksw4, 1.0, true);
-        if (step == nstep) {
-            general::copy(d, st[S_UP], w[W_UP], s);
-            general::copy(d, st[S_VP], w[W_VP], s);
-            general::copy(d, st[S_SSHP], w[W_SSHP], s);
-            general::copy(d, st[S_U], w[W_U], s);
-            general::copy(d, st[S_V], w[W_V], s);
-            general::copy(d, st[S_SSH], w[W_SSH], s);
-        }
+    double **w = c->work, **st = c->state, **h = c->depth, **x = c->scr;
+    const int pairs[6][2] = {{W_UP, S_UP}, {W_VP, S_VP}, {W_SSHP, S_SSHP}, {W_U, S_U}, {W_V, S_V}, {W_SSH, S_SSH}};
+    general::FieldSet begin = {}, save = {};
+    for (const auto &p : pairs) {
+        begin.add(w[p[0]], st[p[1]]);
+        save.add(st[p[1]], w[p[0]]);
     }
-    general::halo(d, c->acc[A_UI], s);
-    general::halo(d, c->acc[A_VI], s);
+    for (int k : {W_UN, W_VN, W_SSHN}) begin.add(w[k], nullptr);
+    for (int k = 0; k < NACC; k++) begin.add(c->acc[k], nullptr);
+    if (ksw4 > 0) {
+        begin.add(x[C_FX], nullptr);
+        begin.add(x[C_FY], nullptr);
+    }
+    general::set_fields(d, begin, s);
+    if (c->c.ffs > 0)
+        general::wrap_fields(d, {x[C_VORT], x[C_STRT], x[C_STRS], h[H_UN], h[H_VN], h[H_HN]}, s);
+    else
+        general::wrap_fields(d, {x[C_VORT], x[C_STRT], x[C_STRS]}, s);
+    general::StepArgs a = step_args(c, w, tau / (double)nstep, nstep);
+    for (int step = 1; step <= 2 * nstep; step++) {
+        a.last = step == 2 * nstep;
+        general::substep(d, c->gdev(), c->c, a, true, false, ksw4, s);
+        if (step == nstep) general::set_fields(d, save, s);
+    }
+    general::wrap_fields(d, {c->acc[A_UI], c->acc[A_VI]}, s);
     if (c->c.ffs > 0) depths_from_state(c);
+}
+
+// nsub calls of barotropic_dynamics(dt, 1) keeping *_e: the first substep
+// of each call, run in place on the saved state, followed by the hh_init
+// that ends every call (its depths are derived in the next substep, and
+// stored after the last)
+void general_run(inmsom_ctx *c, int nsub, double dt, const double *rhs_scale)
+{
+    const Dom &d = c->dom;
+    cudaStream_t s = c->stream;
+    double **st = c->state, **h = c->depth, **x = c->scr;
+    double *w[NWORK];
+    for (int k = 0; k < NWORK; k++) w[k] = c->work[k];
+    w[W_U] = st[S_U]; w[W_UP] = st[S_UP]; w[W_V] = st[S_V]; w[W_VP] = st[S_VP];
+    w[W_SSH] = st[S_SSH]; w[W_SSHP] = st[S_SSHP];
+    if (!c->depths_current) depths_from_state(c);
+    if (nsub < 1) return;
+    general::FieldSet zero = {};
+    for (int k : {W_UN, W_VN, W_SSHN}) zero.add(w[k], nullptr);
+    general::set_fields(d, zero, s);
+    general::wrap_fields(d, {x[C_VORT], x[C_STRT], x[C_STRS]}, s);
+    general::StepArgs a = step_args(c, w, dt, 1);
+    const bool moving = c->c.ffs > 0;
+    for (int k = 0; k < nsub; k++) {
+        if (k == 1 && moving) general::wrap_fields(d, {h[H_U], h[H_V], h[H_H]}, s);
+        a.rhs_scale = rhs_scale ? rhs_scale[k] : 1.0;
+        a.last = k == nsub - 1;
+        general::substep(d, c->gdev(), c->c, a, false, moving && k > 0, 0, s);
+    }
+    if (moving) depths_from_state(c);
 }
 
 int ensure_grid(inmsom_ctx *c)
@@ -444,7 +458,7 @@ int inmsom_barotropic_dynamics(inmsom_ctx *c, double tau, int nstep, int ksw4, d
     }
     CK(cudaEventRecord(c->ph[1], c->stream));
     const bool fused_run = c->fused_ok && ksw4 <= 0;
-    // the fused path derives the depths from SSH; the per-loop path reads them
+    // the fused path derives the depths from SSH; the general path reads them
     if (!c->depths_current && !fused_run) depths_from_state(c);
 
     int rc = INMSOM_OK;
@@ -455,7 +469,7 @@ int inmsom_barotropic_dynamics(inmsom_ctx *c, double tau, int nstep, int ksw4, d
                            cudaGetErrorString(cudaGetLastError()));
         if (c->plan.last_flags & (fused::FLAG_TIMEOUT | fused::FLAG_SMEM)) return fused_flag_error(c, "fused kernel");
         // the call ends with hh_init(ssh_e, sshp_e) (vel_ssh.f90:668-675):
-        // resident depths are derived when next read (per-loop path, diag,
+        // resident depths are derived when next read (general path, diag,
         // sync_to_host), host depths now
         if (c->c.ffs > 0) {
             if (resident) c->depths_current = false;
@@ -686,24 +700,8 @@ int inmsom_run_substeps(inmsom_ctx *c, int nsub, double dt, const double *rhs_sc
         c->depths_current = false;
         if (c->plan.last_flags & (fused::FLAG_TIMEOUT | fused::FLAG_SMEM)) return fused_flag_error(c, "fused kernel");
     } else {
-        // nsub calls of barotropic_dynamics(dt, 1) keeping *_e: the first
-        // substep of each call, run in place on the saved state, followed by
-        // the hh_init that ends every call
-        const Dom &d = c->dom;
-        double **w = c->work, **st = c->state;
-        double *saved[NWORK];
-        for (int k = 0; k < NWORK; k++) saved[k] = w[k];
-        w[W_U] = st[S_U]; w[W_UP] = st[S_UP]; w[W_V] = st[S_V]; w[W_VP] = st[S_VP];
-        w[W_SSH] = st[S_SSH]; w[W_SSHP] = st[S_SSHP];
-        general::fill(d, w[W_UN], 0.0, c->stream);
-        general::fill(d, w[W_VN], 0.0, c->stream);
-        general::fill(d, w[W_SSHN], 0.0, c->stream);
-        if (!c->depths_current) depths_from_state(c);
-        for (int k = 0; k < nsub; k++) {
-            general_substep(c, dt, 1, 0, rhs_scale ? rhs_scale[k] : 1.0, false);
-            if (c->c.ffs > 0) depths_from_state(c);
-        }
-        for (int k = 0; k < NWORK; k++) w[k] = saved[k];
+        general_run(c, nsub, dt, rhs_scale);
+        CK(cudaGetLastError());
     }
     if (!ev1_recorded) CK(cudaEventRecord(c->ev1, c->stream));
     CKR(sync_stream(c));
@@ -896,13 +894,11 @@ int inmsom_ssh_internal(inmsom_ctx *c, double tau, double *ssh_i, double *sshp_i
     const Dom &d = c->dom;
     const GridDev g = c->gdev();
     general::fill(d, I[I_NEW], 0.0, c->stream);  // vel_ssh.f90:704-705
-    general::continuity(d, g, c->c, tau, I[I_NEW], I[I_SSHP], I[I_U], I[I_V], nullptr, nullptr,
-                        I[I_WFLUX], c->stream);
+    general::continuity(d, g, c->c, tau, I[I_NEW], I[I_SSHP], I[I_U], I[I_V], I[I_WFLUX], c->stream);
     general::halo(d, I[I_NEW], c->stream);
     if (c->c.ffs > 0)
         general::hh_update(d, g, I[I_HQN], I[I_HUN], I[I_HVN], I[I_HHN], I[I_NEW], c->stream);
-    general::asselin3(d, g, c->c, 1.0, I[I_SSH], I[I_SSHP], I[I_NEW], nullptr, nullptr, nullptr,
-                      nullptr, nullptr, nullptr, c->stream);
+    general::asselin_ssh(d, g, c->c, I[I_SSH], I[I_SSHP], I[I_NEW], c->stream);
     CKR(d2h(c, ssh_i, I[I_SSH]));
     CKR(d2h(c, sshp_i, I[I_SSHP]));
     for (int k = 0; k < 4; k++) CKR(d2h(c, hi[k], I[I_HQN + k]));

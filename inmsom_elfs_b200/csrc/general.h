@@ -1,12 +1,15 @@
-// Per-loop kernels of the barotropic step ("general path").
+// The barotropic step's general path.
 //
-// One kernel per loop of the reference routines, over the same index
-// ranges, with the same masks and the same expression order; the file is
-// compiled with --fmad=false, so every product and sum rounds where the
-// Fortran expression rounds it.  This path handles everything the reference
-// supports on one domain: 2-D metric arrays, periodic x/y wrap, the
-// biharmonic option (ksw4) and ocean points in the halo ring.
+// The reference's loops over the same index ranges, with the same masks and
+// the same expression order, merged into the few kernels that their
+// dependences allow; the file is compiled with --fmad=false, so every
+// product and sum rounds where the Fortran expression rounds it.  This path
+// handles everything the reference supports on one domain: 2-D metric
+// arrays, periodic x/y wrap, the biharmonic option (ksw4) and ocean points
+// in the halo ring.
 #pragma once
+
+#include <initializer_list>
 
 #include "common.cuh"
 
@@ -15,61 +18,56 @@ namespace general {
 
 // whole-array helpers
 void fill(const Dom &d, double *f, double v, cudaStream_t s);
-void copy(const Dom &d, double *dst, const double *src, cudaStream_t s);
+// dst[k] = src[k], or 0 where src[k] is null, k < n, in one launch
+struct FieldSet {
+    double *dst[16];
+    const double *src[16];
+    int n;
+    void add(double *d, const double *s) { dst[n] = d; src[n++] = s; }
+};
+void set_fields(const Dom &d, const FieldSet &f, cudaStream_t s);
 // syncborder_real8 (a no-op on one domain) + cyclize8_x/_y
 void halo(const Dom &d, double *f, cudaStream_t s);
 
-// Function/depth.f90:2-105
-void hh_init(const Dom &d, const GridDev &g, const Consts &c,
-             double *hq, double *hqp, double *hqn, double *hu, double *hup,
-             double *hun, double *hv, double *hvp, double *hvn, double *hh,
-             double *hhp, double *hhn, const double *sh, const double *shp,
-             cudaStream_t s);
+// the same wraps of up to twelve fields in one launch (none: nothing)
+void wrap_fields(const Dom &d, std::initializer_list<double *> fields, cudaStream_t s);
+
+// Function/depth.f90:2-105; h: hq hqp hqn hu hup hun hv hvp hvn hh hhp hhn
+void hh_init(const Dom &d, const GridDev &g, const Consts &c, double *const h[12], const double *sh,
+             const double *shp, cudaStream_t s);
 // Function/depth.f90:108-170
 void hh_update(const Dom &d, const GridDev &g, double *hqn, double *hun,
                double *hvn, double *hhn, const double *sh, cudaStream_t s);
-// Function/depth.f90:174-220
-void hh_shift(const Dom &d, const GridDev &g, const Consts &c, double *const h[12],
-              int nstep, cudaStream_t s);
-// Function/mixing.f90:115-168
-void stress_components(const Dom &d, const GridDev &g, const double *u,
-                       const double *v, double *str_t, double *str_s,
-                       cudaStream_t s);
-// Function/vel_ssh.f90:2-114
-void uv_trans(const Dom &d, const GridDev &g, const double *u, const double *v,
-              double *vort, const double *hu, const double *hv,
-              const double *hh, double *rhsx, double *rhsy, cudaStream_t s);
-// Function/vel_ssh.f90:117-184
-void uv_diff2(const Dom &d, const GridDev &g, const double *mu,
-              const double *str_t, const double *str_s, const double *hq,
-              const double *hh, double *rhsx, double *rhsy, cudaStream_t s);
-// Function/vel_ssh.f90:187-317
-void uv_diff4(const Dom &d, const GridDev &g, const double *mu, double *str_t,
-              double *str_s, double *fx, double *fy, const double *hq,
-              const double *hu, const double *hv, const double *hh,
-              double *rhsx, double *rhsy, cudaStream_t s);
 
-// Function/vel_ssh.f90:487-499 (and :707-719 with hu = hv = NULL)
+// One substep of the loop body of Function/vel_ssh.f90:484-615 on the work
+// arrays.  means: a substep of barotropic_dynamics (time means, the new
+// depths carried on and shifted by hh_shift); else one of a run, which ends
+// with hh_init of the depths: derive takes the current and previous depths
+// from ssh and sshp (every substep after a run's first) instead of the
+// arrays.  last: store the advective and viscous terms (advx .. dify), which
+// every substep of the reference overwrites.  Before the first substep
+// sshn, un, vn (and fx, fy with ksw4 > 0) are zero and the wraps of vort,
+// strt, strs (and hun, hvn, hhn) are done; before the first derived one
+// those of hu, hv, hh.
+struct StepArgs {
+    double *u, *up, *un, *v, *vp, *vn, *ssh, *sshp, *sshn;
+    double *hq, *hqp, *hqn, *hu, *hup, *hun, *hv, *hvp, *hvn, *hh, *hhp, *hhn;
+    double *vort, *strt, *strs, *fx, *fy, *advx, *advy, *difx, *dify;
+    double *ui, *vi, *gx, *gy;   // time means
+    const double *rhsx, *rhsy, *wflux, *mu, *mu4, *rdis;
+    double rhs_scale;            // RHSx/RHSy are used as RHSx*rhs_scale (x*1.0 == x)
+    double ti, ns, four_nstep;   // inner step, nstep, 4*nstep
+    int last;
+};
+void substep(const Dom &d, const GridDev &g, const Consts &c, const StepArgs &a, bool means, bool derive, int ksw4,
+             cudaStream_t s);
+
+// Function/vel_ssh.f90:707-719 and :738-741 (ssh_internal)
 void continuity(const Dom &d, const GridDev &g, const Consts &c, double dt,
                 double *sshn, const double *sshp, const double *u,
-                const double *v, const double *hu, const double *hv,
-                const double *wflux, cudaStream_t s);
-
-struct MomentumArgs {
-    double *un, *vn, *ubrtr_i, *vbrtr_i, *gx, *gy;
-    const double *u, *v, *up, *vp, *ssh, *sshn;
-    const double *hu, *hup, *hun, *hv, *hvp, *hvn, *hh;
-    const double *rhsx, *rhsy, *difx, *dify, *advx, *advy, *rdis;
-    double rhs_scale;  // RHSx/RHSy are used as RHSx*rhs_scale (x*1.0 == x)
-};
-// Function/vel_ssh.f90:531-573
-void momentum(const Dom &d, const GridDev &g, const Consts &c, double tau_inner,
-              int nstep, const MomentumArgs &a, cudaStream_t s);
-// Function/vel_ssh.f90:589-612 and, with nstep = 1 and u = v = NULL, :738-749
-void asselin3(const Dom &d, const GridDev &g, const Consts &c, double nstep,
-              double *ssh, double *sshp, const double *sshn, double *u,
-              double *up, const double *un, double *v, double *vp,
-              const double *vn, cudaStream_t s);
+                const double *v, const double *wflux, cudaStream_t s);
+void asselin_ssh(const Dom &d, const GridDev &g, const Consts &c, double *ssh, double *sshp, const double *sshn,
+                 cudaStream_t s);
 
 // Control/init_pars.f90:459-481
 void r_diss(const Dom &d, const GridDev &g, double r_fric, double *r, cudaStream_t s);
