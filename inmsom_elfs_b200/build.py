@@ -32,11 +32,12 @@ SOURCES = {
     "closure.cu": [],
     "closure_tc.cu": [],
     "column.cu": ["--fmad=false"],
+    "transfer.cu": [],
     "dstd.cu": [],
     "ctl_read.cu": [],
     "ocean_cp.cu": [],
 }
-HEADERS = ["common.cuh", "general.h", "fused.h", "closure.h", "column.h", "context.h", "gelu.cuh"]
+HEADERS = ["common.cuh", "general.h", "fused.h", "closure.h", "column.h", "transfer.h", "context.h", "gelu.cuh"]
 
 
 def nvcc() -> str:

@@ -295,6 +295,9 @@ int inmsom_gpu_finalize(inmsom_ctx *c)
     cudaFree(c->col_lev);
     cudaFree(c->trc);
     cudaFree(c->trc_lev);
+    transfer::release(c->stage);
+    transfer::release(c->stage_up);
+    transfer::release(c->stage_dn);
     for (auto &e : c->bev)
         if (e) cudaEventDestroy(e);
     if (c->s_up) cudaStreamDestroy(c->s_up);
@@ -345,18 +348,20 @@ int inmsom_gpu_register_grid(inmsom_ctx *c, const float *lu, const float *luu, c
     if (ndepth != 0 && ndepth != NDEPTH)
         return set_err(INMSOM_EARG, "pass all twelve depth arrays or none");
 
+    Copies in(c);
     for (int k = 0; k < NMASK; k++) {
         if (!c->mask[k]) CKR(dalloc(c, &c->mask[k], sizeof(float)));
-        CKR(h2d(c, c->mask[k], hm[k]));
+        CKR(in.add(c->mask[k], hm[k]));
     }
     c->h_lu.assign(lu, lu + (size_t)c->dom.nxa() * c->dom.nya());
     CKR(alloc_set(c, c->met, NMET));
-    for (int k = 0; k < NMET; k++) CKR(h2d(c, c->met[k], hg[k]));
+    for (int k = 0; k < NMET; k++) CKR(in.add(c->met[k], hg[k]));
     CKR(alloc_set(c, c->depth, NDEPTH));
     for (int k = 0; k < NDEPTH; k++) {
         c->h_depth[k] = hd[k];
-        if (hd[k]) CKR(h2d(c, c->depth[k], (const double *)hd[k]));
+        if (hd[k]) CKR(in.add(c->depth[k], (const double *)hd[k]));
     }
+    CKR(in.up());
     c->depths_current = ndepth == NDEPTH;
     CKR(alloc_block(c, c->state, NSTATE));
     CKR(alloc_set(c, c->work, NWORK));
@@ -433,29 +438,36 @@ int inmsom_barotropic_dynamics(inmsom_ctx *c, double tau, int nstep, int ksw4, d
     c->ph_direct = false;
     CK(cudaEventRecord(c->ph[0], c->stream));
 
-    if (!resident || !c->state_on_device) {
-        for (int k = 0; k < NSTATE; k++) CKR(h2d(c, c->state[k], (const double *)hs[k]));
-        c->state_on_device = true;
-        fused::mark_state_changed(c->plan);
-    }
-    if (!resident || !c->scratch_on_device) {
-        for (int k = 0; k < NSCR; k++) CKR(h2d(c, c->scr[k], (const double *)hc[k]));
-        c->scratch_on_device = true;
-    }
+    Copies in(c);
+    const bool new_state = !resident || !c->state_on_device, new_scratch = !resident || !c->scratch_on_device;
+    if (new_state)
+        for (int k = 0; k < NSTATE; k++) CKR(in.add(c->state[k], (const double *)hs[k]));
+    if (new_scratch)
+        for (int k = 0; k < NSCR; k++) CKR(in.add(c->scr[k], (const double *)hc[k]));
     const bool static_coef = resident && (c->flags & INMSOM_STATIC_COEFFS);
     for (int k = 0; k < NFORC; k++) {
         if (k == F_MU4 && ksw4 <= 0) continue;   // read only by uv_diff4
         const bool coef = k != F_RHSX && k != F_RHSY;
         if (static_coef && coef && c->coef_on_device[k]) continue;
-        CKR(h2d(c, c->forc[k], hf[k]));
+        CKR(in.add(c->forc[k], hf[k]));
+    }
+    if (!resident)
+        for (int k = 0; k < NDEPTH; k++)
+            if (c->h_depth[k]) CKR(in.add(c->depth[k], (const double *)c->h_depth[k]));
+    CKR(in.up());
+    if (new_state) {
+        c->state_on_device = true;
+        fused::mark_state_changed(c->plan);
+    }
+    c->scratch_on_device = true;
+    for (int k = 0; k < NFORC; k++) {
+        if (k == F_MU4 && ksw4 <= 0) continue;
+        const bool coef = k != F_RHSX && k != F_RHSY;
+        if (static_coef && coef && c->coef_on_device[k]) continue;
         c->coef_on_device[k] = static_coef && coef;
         c->forc_gen++;
     }
-    if (!resident) {
-        for (int k = 0; k < NDEPTH; k++)
-            if (c->h_depth[k]) CKR(h2d(c, c->depth[k], (const double *)c->h_depth[k]));
-        if (c->h_depth[0]) c->depths_current = true;
-    }
+    if (!resident && c->h_depth[0]) c->depths_current = true;
     CK(cudaEventRecord(c->ph[1], c->stream));
     const bool fused_run = c->fused_ok && ksw4 <= 0;
     // the fused path derives the depths from SSH; the general path reads them
@@ -480,13 +492,15 @@ int inmsom_barotropic_dynamics(inmsom_ctx *c, double tau, int nstep, int ksw4, d
     }
 
     CK(cudaEventRecord(c->ph[2], c->stream));
-    for (int k = 0; k < NACC; k++) CKR(d2h(c, ha[k], c->acc[k]));
+    Copies out(c);
+    for (int k = 0; k < NACC; k++) CKR(out.add(c->acc[k], (const double *)ha[k]));
     if (!resident) {
-        for (int k = 0; k < NSTATE; k++) CKR(d2h(c, hs[k], c->state[k]));
-        for (int k = 0; k < NSCR; k++) CKR(d2h(c, hc[k], c->scr[k]));
+        for (int k = 0; k < NSTATE; k++) CKR(out.add(c->state[k], (const double *)hs[k]));
+        for (int k = 0; k < NSCR; k++) CKR(out.add(c->scr[k], (const double *)hc[k]));
         for (int k = 0; k < NDEPTH; k++)
-            if (c->h_depth[k]) CKR(d2h(c, c->h_depth[k], c->depth[k]));
+            if (c->h_depth[k]) CKR(out.add(c->depth[k], (const double *)c->h_depth[k]));
     }
+    CKR(out.down());
     CK(cudaEventRecord(c->ph[3], c->stream));
     CKR(sync_stream(c));
     c->ph_valid = true;
@@ -522,17 +536,19 @@ int inmsom_load_state(inmsom_ctx *c, double *ubrtr_e, double *ubrtrp_e, double *
     CKR(ensure_grid(c));
     double *hs[NSTATE] = {ubrtr_e, ubrtrp_e, vbrtr_e, vbrtrp_e, ssh_e, sshp_e};
     const double *hf[NFORC] = {RHSx, RHSy, wflux, mu, mu4, rdis};
+    Copies in(c);
     for (int k = 0; k < NSTATE; k++) {
-        CKR(h2d(c, c->state[k], (const double *)hs[k]));
+        CKR(in.add(c->state[k], (const double *)hs[k]));
         c->h_state[k] = hs[k];
     }
     const bool static_coef = (c->flags & INMSOM_RESIDENT) && (c->flags & INMSOM_STATIC_COEFFS);
     for (int k = 0; k < NFORC; k++) {
         if (k == F_MU4 && !mu4) continue;
-        CKR(h2d(c, c->forc[k], hf[k]));
+        CKR(in.add(c->forc[k], hf[k]));
         c->coef_on_device[k] = static_coef && k != F_RHSX && k != F_RHSY;
         c->forc_gen++;
     }
+    CKR(in.up());
     c->state_on_device = true;
     fused::mark_state_changed(c->plan);
     if (c->fused_ok || !c->depths_current) depths_from_state(c);
@@ -1074,17 +1090,19 @@ int inmsom_gpu_diag(inmsom_ctx *c, double *volume, double *energy)
 int inmsom_gpu_sync_to_host(inmsom_ctx *c, unsigned what)
 {
     CKR(ensure_grid(c));
+    Copies out(c);
     if (what & INMSOM_SYNC_STATE) {
         if (!c->state_on_device) return set_err(INMSOM_EARG, "no resident state");
-        for (int k = 0; k < NSTATE; k++) CKR(d2h(c, c->h_state[k], c->state[k]));
+        for (int k = 0; k < NSTATE; k++) CKR(out.add(c->state[k], (const double *)c->h_state[k]));
     }
     if (what & INMSOM_SYNC_DEPTHS) {
         if (!c->depths_current) depths_from_state(c);
         for (int k = 0; k < NDEPTH; k++)
-            if (c->h_depth[k]) CKR(d2h(c, c->h_depth[k], c->depth[k]));
+            if (c->h_depth[k]) CKR(out.add(c->depth[k], (const double *)c->h_depth[k]));
     }
     if (what & INMSOM_SYNC_SCRATCH)
-        for (int k = 0; k < NSCR; k++) CKR(d2h(c, c->h_scr[k], c->scr[k]));
+        for (int k = 0; k < NSCR; k++) CKR(out.add(c->scr[k], (const double *)c->h_scr[k]));
+    CKR(out.down());
     return sync_stream(c);
 }
 
@@ -1092,7 +1110,9 @@ int inmsom_gpu_sync_from_host(inmsom_ctx *c, unsigned what)
 {
     CKR(ensure_grid(c));
     if (what & INMSOM_SYNC_STATE) {
-        for (int k = 0; k < NSTATE; k++) CKR(h2d(c, c->state[k], (const double *)c->h_state[k]));
+        Copies in(c);
+        for (int k = 0; k < NSTATE; k++) CKR(in.add(c->state[k], (const double *)c->h_state[k]));
+        CKR(in.up());
         c->state_on_device = true;
         fused::mark_state_changed(c->plan);
         if (c->fused_ok) c->depths_current = false;

@@ -41,68 +41,25 @@ int col_alloc(inmsom_ctx *c, int nz)
     return INMSOM_OK;
 }
 
-// nlev levels of a host array (bnd_x1:bnd_x2, bnd_y1:bnd_y2, nlev): the
-// host rows of consecutive levels follow each other, as do the device rows
-int h2d3(inmsom_ctx *c, double *dev, const double *host, int nlev)
-{
-    if (!host) return set_err(INMSOM_EARG, "NULL host array");
-    const size_t w = (size_t)c->dom.nxa() * sizeof(double);
-    CK(cudaMemcpy2DAsync(dev + c->dom.xoff, (size_t)c->dom.pitch * sizeof(double), host, w, w,
-                         (size_t)c->dom.nya() * nlev, cudaMemcpyHostToDevice, c->stream));
-    return INMSOM_OK;
-}
-
-int d2h3(inmsom_ctx *c, double *host, const double *dev, int nlev)
-{
-    const size_t w = (size_t)c->dom.nxa() * sizeof(double);
-    CK(cudaMemcpy2DAsync(host, w, dev + c->dom.xoff, (size_t)c->dom.pitch * sizeof(double), w,
-                         (size_t)c->dom.nya() * nlev, cudaMemcpyDeviceToHost, c->stream));
-    return INMSOM_OK;
-}
-
-// rows r0..r1 and array columns x0..x1 (0-based from bnd_x1 / bnd_y1) of
-// nlev levels between a host array (bnd_x1:bnd_x2, bnd_y1:bnd_y2, nlev) and
-// its pitched device copy, as one 3-D copy
-int box3(inmsom_ctx *c, double *dev, double *host, int nlev, int r0, int r1, int x0, int x1, bool up,
-         cudaStream_t s)
-{
-    if (r1 < r0 || x1 < x0) return INMSOM_OK;
-    const Dom &d = c->dom;
-    cudaMemcpy3DParms p = {};
-    cudaPitchedPtr hp = make_cudaPitchedPtr(host, (size_t)d.nxa() * sizeof(double), (size_t)d.nxa(), (size_t)d.nya());
-    cudaPitchedPtr dp = make_cudaPitchedPtr(dev + d.xoff, (size_t)d.pitch * sizeof(double), (size_t)d.nxa(),
-                                            (size_t)d.nya());
-    const cudaPos pos = make_cudaPos((size_t)x0 * sizeof(double), (size_t)r0, 0);
-    p.srcPtr = up ? hp : dp;
-    p.dstPtr = up ? dp : hp;
-    p.srcPos = pos;
-    p.dstPos = pos;
-    p.extent = make_cudaExtent((size_t)(x1 - x0 + 1) * sizeof(double), (size_t)(r1 - r0 + 1), (size_t)nlev);
-    p.kind = up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-    CK(cudaMemcpy3DAsync(&p, s));
-    return INMSOM_OK;
-}
-
-// A 3-D field of a banded call: its device copy, the host array, its levels
-struct Field3 {
-    double *dev;
-    double *host;
-    int nlev;
-};
+using transfer::Field;
 
 // The copy pipeline of the 3-D entry points.  The interior rows are cut into
 // nb bands; band b's rows of the inputs are uploaded on s_up while band b-1
-// runs on the context's stream (run(n0, n1)) and band b-2's interior
+// runs on the context's stream (run(n0, n1), then sides(n0, n1) for those
+// rows' points west and east of the interior) and band b-2's rows of the
 // results go back on s_dn.  Each input row is uploaded once: band b brings
 // the rows from just after band b-1's last to one past its own last
 // interior row (run reads rows n0-1..n1+1), the last band the rest of the
-// arrays.  After every band, border() runs and everything of the outputs
-// outside the interior is downloaded.  pre(s_up) issues the 2-D uploads;
-// flag (4 bytes on the device) is read back at the end.  The phase times
-// are the uploads, the kernels' own time (CUDA events around each run and
-// the border) and from the last kernel to the end.
-int pipelined(inmsom_ctx *c, int nb, const std::vector<Field3> &in, const std::vector<Field3> &out,
-              const std::function<int(cudaStream_t)> &pre, const std::function<int(int, int)> &run,
+// arrays.  After every band, border() computes the rows south and north of
+// the interior, and they are downloaded.  pre holds the 2-D inputs, lev the
+// levels' dz and hzt (2 nz + 1 doubles on the device); flag (4 bytes on the
+// device) is read back at the end.  The phase times are the uploads, the
+// kernels' own time (CUDA events around each run and the border) and from
+// the last kernel to the end.  Whole rows go both ways: a side's two columns
+// by themselves were rows of 16 bytes to the copy engine, 0.1 us each.
+int pipelined(inmsom_ctx *c, int nb, const std::vector<Field> &pre, const double *dz, const double *hzt, int nz,
+              double *lev, const std::vector<Field> &in, const std::vector<Field> &out,
+              const std::function<int(int, int)> &run, const std::function<int(int, int)> &sides,
               const std::function<int()> &border, const int *flag_dev, int *flag)
 {
     const Dom &d = c->dom;
@@ -113,43 +70,46 @@ int pipelined(inmsom_ctx *c, int nb, const std::vector<Field3> &in, const std::v
     cudaEvent_t *ev_up = c->bev, *ev_k0 = c->bev + 8, *ev_k1 = c->bev + 16, *ev_bd = c->bev + 32;
     const int nyi = d.ny_end - d.ny_start + 1;
     nb = std::max(1, std::min(nb, std::min(8, nyi)));
-    const int nxa = d.nxa(), nya = d.nya();
-    const int ix0 = d.nx_start - d.bnd_x1, ix1 = d.nx_end - d.bnd_x1;      // interior, 0-based
+    const int nya = d.nya();
     const int iy0 = d.ny_start - d.bnd_y1, iy1 = d.ny_end - d.bnd_y1;
+    auto failed = [] { return set_err(INMSOM_ECUDA, "launch failed: %s", cudaGetErrorString(cudaGetLastError())); };
+    auto up = [&](const std::vector<Field> &f, int r0, int r1) {
+        return transfer::rows(c->stage_up, d, f.data(), (int)f.size(), r0, r1, true, c->s_up);
+    };
+    auto down = [&](int r0, int r1) {
+        return transfer::rows(c->stage_dn, d, out.data(), (int)out.size(), r0, r1, false, c->s_dn);
+    };
     c->ph_valid = false;
     c->ph_direct = false;
     CK(cudaEventRecord(c->ph[0], c->stream));
     CK(cudaStreamWaitEvent(c->s_up, c->ph[0], 0));
-    CKR(pre(c->s_up));
+    CK(cudaMemcpyAsync(lev, dz, nz * sizeof(double), cudaMemcpyHostToDevice, c->s_up));
+    CK(cudaMemcpyAsync(lev + nz, hzt, (nz + 1) * sizeof(double), cudaMemcpyHostToDevice, c->s_up));
+    CK(up(pre, 0, nya - 1));
     int up_next = 0;
     for (int b = 0; b < nb; b++) {
         const int n0 = d.ny_start + (int)((long long)nyi * b / nb);
         const int n1 = d.ny_start + (int)((long long)nyi * (b + 1) / nb) - 1;
         const int up_last = b == nb - 1 ? nya - 1 : n1 + 1 - d.bnd_y1;
-        for (const Field3 &f : in) CKR(box3(c, f.dev, f.host, f.nlev, up_next, up_last, 0, nxa - 1, true, c->s_up));
+        CK(up(in, up_next, up_last));
         up_next = up_last + 1;
         CK(cudaEventRecord(ev_up[b], c->s_up));
         CK(cudaStreamWaitEvent(c->stream, ev_up[b], 0));
         CK(cudaEventRecord(ev_k0[b], c->stream));
-        if (run(n0, n1)) return set_err(INMSOM_ECUDA, "launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+        if (run(n0, n1) || sides(n0, n1)) return failed();
         CK(cudaGetLastError());
         CK(cudaEventRecord(ev_k1[b], c->stream));
         CK(cudaStreamWaitEvent(c->s_dn, ev_k1[b], 0));
-        for (const Field3 &f : out)
-            CKR(box3(c, f.dev, f.host, f.nlev, n0 - d.bnd_y1, n1 - d.bnd_y1, ix0, ix1, false, c->s_dn));
+        CK(down(n0 - d.bnd_y1, n1 - d.bnd_y1));
     }
     CK(cudaEventRecord(ev_bd[0], c->stream));
-    if (border()) return set_err(INMSOM_ECUDA, "launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+    if (border()) return failed();
     CK(cudaGetLastError());
     CK(cudaEventRecord(ev_bd[1], c->stream));
     CK(cudaStreamWaitEvent(c->s_dn, ev_bd[1], 0));
     CK(cudaMemcpyAsync(flag, flag_dev, sizeof(int), cudaMemcpyDeviceToHost, c->s_dn));
-    for (const Field3 &f : out) {
-        CKR(box3(c, f.dev, f.host, f.nlev, 0, iy0 - 1, 0, nxa - 1, false, c->s_dn));             // rows above
-        CKR(box3(c, f.dev, f.host, f.nlev, iy1 + 1, nya - 1, 0, nxa - 1, false, c->s_dn));       // rows below
-        CKR(box3(c, f.dev, f.host, f.nlev, iy0, iy1, 0, ix0 - 1, false, c->s_dn));              // columns left
-        CKR(box3(c, f.dev, f.host, f.nlev, iy0, iy1, ix1 + 1, nxa - 1, false, c->s_dn));        // columns right
-    }
+    CK(down(0, iy0 - 1));
+    CK(down(iy1 + 1, nya - 1));
     CK(cudaEventRecord(c->ph[3], c->s_dn));
     CK(cudaStreamWaitEvent(c->stream, c->ph[3], 0));
     CKR(sync_stream(c));
@@ -220,25 +180,19 @@ int inmsom_baroclinic_dynamics(inmsom_ctx *c, int nz, const double *dz, const do
     // the nz-level inputs in the order of the block's fields C3_UU .. C3_RHSYT
     double *const up3[8] = {uu, uup, vv, vvp, (double *)RHSx, (double *)RHSy, (double *)RHSx_tran,
                             (double *)RHSy_tran};
-    std::vector<Field3> in, out;
-    for (int k = 0; k < 8; k++) in.push_back({col3(c, C3_UU + k), up3[k], nz});
-    in.push_back({colw(c, 0), (double *)ww, nz + 1});
-    in.push_back({colw(c, 1), (double *)nu, nz + 1});
-    for (int k = 0; k < 4; k++) out.push_back({col3(c, C3_UUO + k), io[k], nz});
+    constexpr int F8 = (int)sizeof(double);
+    std::vector<Field> pre, in, out;
+    for (int k = 0; k < NC2; k++) pre.push_back({col2(c, k), (void *)in2[k], 1, F8});
+    for (int k = 0; k < 8; k++) in.push_back({col3(c, C3_UU + k), up3[k], nz, F8});
+    in.push_back({colw(c, 0), (void *)ww, nz + 1, F8});
+    in.push_back({colw(c, 1), (void *)nu, nz + 1, F8});
+    for (int k = 0; k < 4; k++) out.push_back({col3(c, C3_UUO + k), io[k], nz, F8});
     CK(cudaMemsetAsync(a.flag, 0, sizeof(int), c->stream));
-    auto pre = [&](cudaStream_t su) -> int {
-        for (int k = 0; k < NC2; k++)
-            CK(cudaMemcpy2DAsync(col2(c, k) + d.xoff, (size_t)d.pitch * sizeof(double), in2[k],
-                                 d.nxa() * sizeof(double), d.nxa() * sizeof(double), d.nya(),
-                                 cudaMemcpyHostToDevice, su));
-        CK(cudaMemcpyAsync(c->col_lev, dz, nz * sizeof(double), cudaMemcpyHostToDevice, su));
-        CK(cudaMemcpyAsync(c->col_lev + nz, hzt, (nz + 1) * sizeof(double), cudaMemcpyHostToDevice, su));
-        return INMSOM_OK;
-    };
     auto run = [&](int n0, int n1) { return column::baroclinic_rows(d, gd, c->c, L, a, n0, n1, c->stream); };
+    auto sides = [&](int n0, int n1) { return column::baroclinic_sides(d, gd, c->c, L, a, n0, n1, c->stream); };
     auto border = [&]() { return column::baroclinic_border(d, gd, c->c, L, a, c->stream); };
     int flag = 0;
-    CKR(pipelined(c, 8, in, out, pre, run, border, a.flag, &flag));
+    CKR(pipelined(c, 8, pre, dz, hzt, nz, c->col_lev, in, out, run, sides, border, a.flag, &flag));
     if (flag) return set_err(INMSOM_ETIMEOUT, "inmsom_baroclinic_dynamics: a bounded wait of the column kernel gave up");
     c->ph_valid = true;
     return INMSOM_OK;
@@ -338,32 +292,24 @@ int inmsom_tracer_tran_diff(inmsom_ctx *c, int nz, const double *dz, const doubl
     const GridDev gd = c->gdev();
     const int f3[6] = {T_FF, T_FFP, T_UU, T_VV, T_MU, T_SRC};
     const int f31[6] = {T_WW, T_NU, T_SLRX, T_SLRY, T_SLZX, T_SLZY};
-    std::vector<Field3> in, out;
-    for (int k = 0; k < 6; k++) in.push_back({trc3(c, f3[k]), (double *)in3[k], nz});
-    for (int k = 0; k < 6; k++) in.push_back({trc31(c, f31[k]), (double *)in31[k], nz + 1});
-    out.push_back({trc3(c, T_FFO), ff, nz});
-    out.push_back({trc3(c, T_FFPO), ffp, nz});
-    out.push_back({trc2(c, T_FFX), flux_f_x, 4});
-    out.push_back({trc2(c, T_FFY), flux_f_y, 4});
+    constexpr int F8 = (int)sizeof(double), I4 = (int)sizeof(int);
+    std::vector<Field> pre, in, out;
+    for (int k = 0; k < 7; k++) pre.push_back({trc2(c, T_TOP + k), (void *)in2[k], 1, F8});
+    pre.push_back({trc2(c, T_IGT), (void *)ig_top, 1, I4});
+    pre.push_back({trc2(c, T_IGB), (void *)ig_bot, 1, I4});
+    for (int k = 0; k < 6; k++) in.push_back({trc3(c, f3[k]), (void *)in3[k], nz, F8});
+    for (int k = 0; k < 6; k++) in.push_back({trc31(c, f31[k]), (void *)in31[k], nz + 1, F8});
+    out.push_back({trc3(c, T_FFO), ff, nz, F8});
+    out.push_back({trc3(c, T_FFPO), ffp, nz, F8});
+    out.push_back({trc2(c, T_FFX), flux_f_x, 4, F8});
+    out.push_back({trc2(c, T_FFY), flux_f_y, 4, F8});
     CK(cudaMemsetAsync(a.flag, 0, sizeof(int), c->stream));
-    auto pre = [&](cudaStream_t su) -> int {
-        const size_t w = (size_t)d.nxa() * sizeof(double), dp = (size_t)d.pitch * sizeof(double);
-        for (int k = 0; k < 7; k++)
-            CK(cudaMemcpy2DAsync(trc2(c, T_TOP + k) + d.xoff, dp, in2[k], w, w, d.nya(), cudaMemcpyHostToDevice, su));
-        const size_t wi = (size_t)d.nxa() * sizeof(int), dpi = (size_t)d.pitch * sizeof(int);
-        CK(cudaMemcpy2DAsync(reinterpret_cast<int *>(trc2(c, T_IGT)) + d.xoff, dpi, ig_top, wi, wi, d.nya(),
-                             cudaMemcpyHostToDevice, su));
-        CK(cudaMemcpy2DAsync(reinterpret_cast<int *>(trc2(c, T_IGB)) + d.xoff, dpi, ig_bot, wi, wi, d.nya(),
-                             cudaMemcpyHostToDevice, su));
-        CK(cudaMemcpyAsync(c->trc_lev, dz, nz * sizeof(double), cudaMemcpyHostToDevice, su));
-        CK(cudaMemcpyAsync(c->trc_lev + nz, hzt, (nz + 1) * sizeof(double), cudaMemcpyHostToDevice, su));
-        return INMSOM_OK;
-    };
     auto run = [&](int n0, int n1) { return column::tracer_rows(d, gd, c->c, L, a, n0, n1, c->stream); };
+    auto sides = [&](int n0, int n1) { return column::tracer_sides(d, gd, c->c, L, a, n0, n1, c->stream); };
     auto border = [&]() { return column::tracer_border(d, gd, c->c, L, a, c->stream); };
     int flag = 0;
     // a periodic y wraps the y-fluxes of every row before any solve: one band
-    CKR(pipelined(c, d.py ? 1 : 8, in, out, pre, run, border, a.flag, &flag));
+    CKR(pipelined(c, d.py ? 1 : 8, pre, dz, hzt, nz, c->trc_lev, in, out, run, sides, border, a.flag, &flag));
     if (flag) return set_err(INMSOM_ETIMEOUT, "inmsom_tracer_tran_diff: a bounded wait of the solve gave up");
     c->ph_valid = true;
     return INMSOM_OK;
@@ -380,19 +326,21 @@ int inmsom_vertical_velocity(inmsom_ctx *c, int nz, const double *dz, const doub
     c->ph_valid = false;
     c->ph_direct = false;
     CK(cudaEventRecord(c->ph[0], c->stream));
-    CKR(h2d3(c, col3(c, C3_UU), u, nz));
-    CKR(h2d3(c, col3(c, C3_VV), v, nz));
-    CKR(h2d3(c, colw(c, 0), w, nz + 1));
-    CKR(h2d(c, col2(c, 0), hu));
-    CKR(h2d(c, col2(c, 1), hv));
-    CKR(h2d(c, col2(c, 2), wflux));
+    Copies q(c);
+    CKR(q.add(col3(c, C3_UU), u, nz));
+    CKR(q.add(col3(c, C3_VV), v, nz));
+    CKR(q.add(colw(c, 0), (const double *)w, nz + 1));
+    CKR(q.add(col2(c, 0), hu));
+    CKR(q.add(col2(c, 1), hv));
+    CKR(q.add(col2(c, 2), wflux));
+    CKR(q.up());
     CK(cudaMemcpyAsync(c->col_lev, dz, nz * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CK(cudaEventRecord(c->ph[1], c->stream));
     column::vertical_velocity(c->dom, c->gdev(), c->c, col_levels(c), col3(c, C3_UU), col3(c, C3_VV), colw(c, 0),
                               col2(c, 0), col2(c, 1), col2(c, 2), c->stream);
     CK(cudaGetLastError());
     CK(cudaEventRecord(c->ph[2], c->stream));
-    CKR(d2h3(c, w, colw(c, 0), nz + 1));
+    CKR(d2h(c, w, colw(c, 0), nz + 1));
     CK(cudaEventRecord(c->ph[3], c->stream));
     CKR(sync_stream(c));
     c->ph_valid = true;
@@ -406,14 +354,17 @@ int inmsom_depth_ave(inmsom_ctx *c, int nz, const double *dz, double *u, double 
     if (!dz || !u || !utr || !mask) return set_err(INMSOM_EARG, "inmsom_depth_ave: NULL argument");
     CKR(col_alloc(c, nz));
     float *dmask = (float *)col2(c, 1);     // a float plane fits in a double one
-    CKR(h2d3(c, col3(c, C3_UU), u, nz));
-    CKR(h2d(c, col2(c, 0), (const double *)utr));
-    CKR(h2d(c, dmask, mask));
+    Copies q(c);
+    CKR(q.add(col3(c, C3_UU), (const double *)u, nz));
+    CKR(q.add(col2(c, 0), (const double *)utr));
+    CKR(q.add(dmask, mask));
+    CKR(q.up());
     CK(cudaMemcpyAsync(c->col_lev, dz, nz * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     column::depth_ave(c->dom, col_levels(c), col3(c, C3_UU), col2(c, 0), dmask, kbcl, c->stream);
     CK(cudaGetLastError());
-    CKR(d2h3(c, u, col3(c, C3_UU), nz));
-    CKR(d2h(c, utr, col2(c, 0)));
+    CKR(q.add(col3(c, C3_UU), (const double *)u, nz));
+    CKR(q.add(col2(c, 0), (const double *)utr));
+    CKR(q.down());
     return sync_stream(c);
 }
 
@@ -425,15 +376,18 @@ int inmsom_shift_barotropic(inmsom_ctx *c, int nz, double *uu, double *vv, const
     if (sign != 1 && sign != -1) return set_err(INMSOM_EARG, "inmsom_shift_barotropic: sign must be +1 or -1");
     if (!uu || !vv || !uu2d || !vv2d) return set_err(INMSOM_EARG, "inmsom_shift_barotropic: NULL argument");
     CKR(col_alloc(c, nz));
-    CKR(h2d3(c, col3(c, C3_UU), uu, nz));
-    CKR(h2d3(c, col3(c, C3_VV), vv, nz));
-    CKR(h2d(c, col2(c, 0), uu2d));
-    CKR(h2d(c, col2(c, 1), vv2d));
+    Copies q(c);
+    CKR(q.add(col3(c, C3_UU), (const double *)uu, nz));
+    CKR(q.add(col3(c, C3_VV), (const double *)vv, nz));
+    CKR(q.add(col2(c, 0), uu2d));
+    CKR(q.add(col2(c, 1), vv2d));
+    CKR(q.up());
     column::shift_barotropic(c->dom, c->gdev(), col_levels(c), col3(c, C3_UU), col3(c, C3_VV), col2(c, 0),
                              col2(c, 1), sign, c->stream);
     CK(cudaGetLastError());
-    CKR(d2h3(c, uu, col3(c, C3_UU), nz));
-    CKR(d2h3(c, vv, col3(c, C3_VV), nz));
+    CKR(q.add(col3(c, C3_UU), (const double *)uu, nz));
+    CKR(q.add(col3(c, C3_VV), (const double *)vv, nz));
+    CKR(q.down());
     return sync_stream(c);
 }
 
@@ -444,16 +398,19 @@ int inmsom_stress_components(inmsom_ctx *c, int nlev, const double *u, const dou
     if (nlev < 1 || nlev > 65535) return set_err(INMSOM_EARG, "inmsom_stress_components: nlev = %d", nlev);
     if (!u || !v || !str_t || !str_s) return set_err(INMSOM_EARG, "inmsom_stress_components: NULL argument");
     CKR(col_alloc(c, nlev));
-    CKR(h2d3(c, col3(c, C3_UU), u, nlev));
-    CKR(h2d3(c, col3(c, C3_VV), v, nlev));
-    CKR(h2d3(c, col3(c, C3_RHSX), str_t, nlev));   // points the routine does not set keep the caller's values
-    CKR(h2d3(c, col3(c, C3_RHSY), str_s, nlev));
+    Copies q(c);
+    CKR(q.add(col3(c, C3_UU), u, nlev));
+    CKR(q.add(col3(c, C3_VV), v, nlev));
+    CKR(q.add(col3(c, C3_RHSX), (const double *)str_t, nlev));   // points the routine does not set keep the caller's values
+    CKR(q.add(col3(c, C3_RHSY), (const double *)str_s, nlev));
+    CKR(q.up());
     if (column::stress_components(c->dom, c->gdev(), col_levels(c), col3(c, C3_UU), col3(c, C3_VV),
                                   col3(c, C3_RHSX), col3(c, C3_RHSY), c->stream))
         return set_err(INMSOM_EARG, "inmsom_stress_components: bad levels");
     CK(cudaGetLastError());
-    CKR(d2h3(c, str_t, col3(c, C3_RHSX), nlev));
-    CKR(d2h3(c, str_s, col3(c, C3_RHSY), nlev));
+    CKR(q.add(col3(c, C3_RHSX), (const double *)str_t, nlev));
+    CKR(q.add(col3(c, C3_RHSY), (const double *)str_s, nlev));
+    CKR(q.down());
     return sync_stream(c);
 }
 
@@ -466,16 +423,19 @@ int inmsom_smagorinsky_coeff(inmsom_ctx *c, int nz, double visc2, double dift, c
     // Inc/basinpar.fi:72,89: Pi, vonkarman
     const double kp = 0.4 / 3.141592653589793;
     CKR(col_alloc(c, nz));
-    CKR(h2d3(c, col3(c, C3_UU), str_t, nz));
-    CKR(h2d3(c, col3(c, C3_VV), str_s, nz));
-    CKR(h2d3(c, col3(c, C3_RHSX), amts, nz));      // land points keep the caller's values
-    CKR(h2d3(c, col3(c, C3_RHSY), amuv, nz));
+    Copies q(c);
+    CKR(q.add(col3(c, C3_UU), str_t, nz));
+    CKR(q.add(col3(c, C3_VV), str_s, nz));
+    CKR(q.add(col3(c, C3_RHSX), (const double *)amts, nz));      // land points keep the caller's values
+    CKR(q.add(col3(c, C3_RHSY), (const double *)amuv, nz));
+    CKR(q.up());
     if (column::smagorinsky_coeff(c->dom, c->gdev(), col_levels(c), visc2, dift, kp, col3(c, C3_UU),
                                   col3(c, C3_VV), col3(c, C3_RHSX), col3(c, C3_RHSY), c->stream))
         return set_err(INMSOM_EARG, "inmsom_smagorinsky_coeff: bad levels");
     CK(cudaGetLastError());
-    CKR(d2h3(c, amts, col3(c, C3_RHSX), nz));
-    CKR(d2h3(c, amuv, col3(c, C3_RHSY), nz));
+    CKR(q.add(col3(c, C3_RHSX), (const double *)amts, nz));
+    CKR(q.add(col3(c, C3_RHSY), (const double *)amuv, nz));
+    CKR(q.down());
     return sync_stream(c);
 }
 

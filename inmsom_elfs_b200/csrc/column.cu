@@ -398,27 +398,28 @@ __device__ __forceinline__ double new_at(const Dom &D, const float *mask, const 
     return mask[j] > 0.5f ? out[lev + j] : 0.0;
 }
 
-// Function/vel_ssh.f90:1002-1024 outside the interior, one level per grid row
-__global__ void k_border(Dom D, GridDev g, Levels L, BaroclinicArgs a, double ts, int count)
+// Point t outside the interior: of the columns west and east of it on the
+// rows from row0, or (row0 < bnd_y1) of the rows south and north of it
+__device__ __forceinline__ void border_point(const Dom &D, int t, int row0, int &m, int &n)
 {
-    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t0 >= count) return;
-    const int nxa = D.bnd_x2 - D.bnd_x1 + 1;
-    const int h0 = D.ny_start - D.bnd_y1, h1 = D.bnd_y2 - D.ny_end;
-    const int w0 = D.nx_start - D.bnd_x1, w1 = D.bnd_x2 - D.nx_end;
-    int m, n, t = t0;
-    if (t < h0 * nxa) {
-        n = D.bnd_y1 + t / nxa;
-        m = D.bnd_x1 + t % nxa;
-    } else if ((t -= h0 * nxa) < h1 * nxa) {
-        n = D.ny_end + 1 + t / nxa;
+    if (row0 < D.bnd_y1) {
+        const int nxa = D.bnd_x2 - D.bnd_x1 + 1, h0 = D.ny_start - D.bnd_y1, r = t / nxa;
+        n = r < h0 ? D.bnd_y1 + r : D.ny_end + 1 + (r - h0);
         m = D.bnd_x1 + t % nxa;
     } else {
-        t -= h1 * nxa;
-        n = D.ny_start + t / (w0 + w1);
-        const int c = t % (w0 + w1);
+        const int w0 = D.nx_start - D.bnd_x1, w = w0 + D.bnd_x2 - D.nx_end, c = t % w;
+        n = row0 + t / w;
         m = c < w0 ? D.bnd_x1 + c : D.nx_end + 1 + (c - w0);
     }
+}
+
+// Function/vel_ssh.f90:1002-1024 outside the interior, one level per grid row
+__global__ void k_border(Dom D, GridDev g, Levels L, BaroclinicArgs a, double ts, int row0, int count)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= count) return;
+    int m, n;
+    border_point(D, t, row0, m, n);
     const long long i = X(m, n);
     const bool ring = m >= D.nx_start - 1 && m <= D.nx_end + 1 && n >= D.ny_start - 1 && n <= D.ny_end + 1;
     const bool fu = ring && g.lcu[i] > 0.5f, fv = ring && g.lcv[i] > 0.5f;
@@ -863,26 +864,12 @@ __global__ void __launch_bounds__(3 * 32) k_tracer_solve(Dom D, GridDev g, Level
 
 // :405-419 outside the interior (the ring with the wrapped new tracer,
 // copies elsewhere), one level per grid row
-__global__ void k_tracer_border(Dom D, GridDev g, Levels L, TracerArgs a, double ts, int count)
+__global__ void k_tracer_border(Dom D, GridDev g, Levels L, TracerArgs a, double ts, int row0, int count)
 {
-    const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t0 >= count) return;
-    const int nxa = D.bnd_x2 - D.bnd_x1 + 1;
-    const int h0 = D.ny_start - D.bnd_y1, h1 = D.bnd_y2 - D.ny_end;
-    const int w0 = D.nx_start - D.bnd_x1, w1 = D.bnd_x2 - D.nx_end;
-    int m, n, t = t0;
-    if (t < h0 * nxa) {
-        n = D.bnd_y1 + t / nxa;
-        m = D.bnd_x1 + t % nxa;
-    } else if ((t -= h0 * nxa) < h1 * nxa) {
-        n = D.ny_end + 1 + t / nxa;
-        m = D.bnd_x1 + t % nxa;
-    } else {
-        t -= h1 * nxa;
-        n = D.ny_start + t / (w0 + w1);
-        const int c = t % (w0 + w1);
-        m = c < w0 ? D.bnd_x1 + c : D.nx_end + 1 + (c - w0);
-    }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= count) return;
+    int m, n;
+    border_point(D, t, row0, m, n);
     const long long i = X(m, n);
     const bool ring = m >= D.nx_start - 1 && m <= D.nx_end + 1 && n >= D.ny_start - 1 && n <= D.ny_end + 1;
     const long long lev = (long long)blockIdx.y * L.plane, o = lev + i;
@@ -1032,20 +1019,19 @@ int baroclinic_rows(const Dom &d, const GridDev &g, const Consts &c, const Level
     return 0;
 }
 
-int baroclinic_border(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const BaroclinicArgs &a,
-                      cudaStream_t s)
+int baroclinic_sides(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const BaroclinicArgs &a, int n0, int n1,
+                 cudaStream_t s)
 {
-    const int nxi = d.nx_end - d.nx_start + 1, nyi = d.ny_end - d.ny_start + 1;
-    const int count = d.nxa() * d.nya() - nxi * nyi;
-    if (count > 0) k_border<<<dim3((count + 127) / 128, L.nz), 128, 0, s>>>(d, g, L, a, c.ts, count);
+    const int count = (n1 - n0 + 1) * (d.nxa() - (d.nx_end - d.nx_start + 1));
+    if (count > 0) k_border<<<dim3((count + 127) / 128, L.nz), 128, 0, s>>>(d, g, L, a, c.ts, n0, count);
     return 0;
 }
 
-int baroclinic_dynamics(const Dom &d, const GridDev &g, const Consts &c, const Levels &L,
-                        const BaroclinicArgs &a, cudaStream_t s)
+int baroclinic_border(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const BaroclinicArgs &a, cudaStream_t s)
 {
-    if (baroclinic_rows(d, g, c, L, a, d.ny_start, d.ny_end, s)) return -1;
-    return baroclinic_border(d, g, c, L, a, s);
+    const int count = d.nxa() * (d.nya() - (d.ny_end - d.ny_start + 1));
+    if (count > 0) k_border<<<dim3((count + 127) / 128, L.nz), 128, 0, s>>>(d, g, L, a, c.ts, d.bnd_y1 - 1, count);
+    return 0;
 }
 
 int tracer_rows(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const TracerArgs &a, int n0, int n1,
@@ -1080,20 +1066,19 @@ int tracer_rows(const Dom &d, const GridDev &g, const Consts &c, const Levels &L
     return 0;
 }
 
-int tracer_border(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const TracerArgs &a,
-                  cudaStream_t s)
+int tracer_sides(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const TracerArgs &a, int n0, int n1,
+                 cudaStream_t s)
 {
-    const int nxi = d.nx_end - d.nx_start + 1, nyi = d.ny_end - d.ny_start + 1;
-    const int count = d.nxa() * d.nya() - nxi * nyi;
-    if (count > 0) k_tracer_border<<<dim3((count + 127) / 128, L.nz), 128, 0, s>>>(d, g, L, a, c.ts, count);
+    const int count = (n1 - n0 + 1) * (d.nxa() - (d.nx_end - d.nx_start + 1));
+    if (count > 0) k_tracer_border<<<dim3((count + 127) / 128, L.nz), 128, 0, s>>>(d, g, L, a, c.ts, n0, count);
     return 0;
 }
 
-int tracer_tran_diff(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const TracerArgs &a,
-                     cudaStream_t s)
+int tracer_border(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const TracerArgs &a, cudaStream_t s)
 {
-    if (tracer_rows(d, g, c, L, a, d.ny_start, d.ny_end, s)) return -1;
-    return tracer_border(d, g, c, L, a, s);
+    const int count = d.nxa() * (d.nya() - (d.ny_end - d.ny_start + 1));
+    if (count > 0) k_tracer_border<<<dim3((count + 127) / 128, L.nz), 128, 0, s>>>(d, g, L, a, c.ts, d.bnd_y1 - 1, count);
+    return 0;
 }
 
 int depth_ave(const Dom &d, const Levels &L, double *u, double *utr, const float *mask, int kbcl, cudaStream_t s)

@@ -45,16 +45,17 @@ int max_levels();
 // would then need the wrapped value at an interior point; not supported)
 bool wrap_inside(const Dom &d);
 
-// Function/vel_ssh.f90:794-1027 on one domain.  Returns 0, or -1 when nz is
-// out of range or a periodic wrap column/row lies inside the interior.
-int baroclinic_dynamics(const Dom &d, const GridDev &g, const Consts &c, const Levels &L,
-                        const BaroclinicArgs &a, cudaStream_t s);
-// The same in parts: the column solves of interior rows n0..n1 (they read
-// the inputs of rows n0-1..n1+1 and write the outputs of those interior
-// rows only), then, after every interior row, the border (the ring's filter
-// with the wrapped new velocity, copies elsewhere).
+// Function/vel_ssh.f90:794-1027 on one domain, in parts: the column solves
+// of interior rows n0..n1 (they read the inputs of rows n0-1..n1+1 and write
+// the outputs of those interior rows only; -1 when nz is out of range or a
+// periodic wrap column/row lies inside the interior), then those rows' sides
+// (the points west and east of the interior: the ring's filter with the
+// wrapped new velocity, copies elsewhere) and, after every interior row, the
+// border (the rows south and north of it).
 int baroclinic_rows(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const BaroclinicArgs &a,
                     int n0, int n1, cudaStream_t s);
+int baroclinic_sides(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const BaroclinicArgs &a, int n0,
+                     int n1, cudaStream_t s);
 int baroclinic_border(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const BaroclinicArgs &a,
                       cudaStream_t s);
 
@@ -81,15 +82,14 @@ struct TracerArgs {
 };
 
 // Function/tem_sal.f90:1-422 on one domain (hhq_rest from the grid's rest
-// depth).  Returns 0, or -1 when nz is out of range or a periodic wrap
-// column/row lies inside the interior.
-int tracer_tran_diff(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const TracerArgs &a,
-                     cudaStream_t s);
-// The same in parts: the fluxes and column solves of interior rows n0..n1
-// (the solves read the fluxes of row n0-1, which an earlier call wrote;
-// with a periodic y the whole interior at once), then the border.
+// depth), in parts as above: the fluxes and column solves of interior rows
+// n0..n1 (the solves read the fluxes of row n0-1, which an earlier call
+// wrote; with a periodic y the whole interior at once), the sides, the
+// border.
 int tracer_rows(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const TracerArgs &a, int n0, int n1,
                 cudaStream_t s);
+int tracer_sides(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const TracerArgs &a, int n0, int n1,
+                 cudaStream_t s);
 int tracer_border(const Dom &d, const GridDev &g, const Consts &c, const Levels &L, const TracerArgs &a,
                   cudaStream_t s);
 

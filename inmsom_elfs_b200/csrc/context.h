@@ -13,6 +13,7 @@
 #include "common.cuh"
 #include "closure.h"
 #include "fused.h"
+#include "transfer.h"
 #include "general.h"
 
 namespace inmsom {
@@ -86,6 +87,7 @@ struct inmsom_ctx {
     cudaEvent_t bev[4 * 8 + 4] = {};
     float ph_ms[3] = {};
     bool ph_direct = false;
+    transfer::Stage stage, stage_up, stage_dn;   // packed rows on their way: on stream, s_up, s_dn
     // inmsom_tracer_tran_diff: fields of trc_nz levels in one block and dz, hzt
     double *trc = nullptr, *trc_lev = nullptr;
     int trc_nz = 0;
@@ -155,24 +157,48 @@ int dalloc(inmsom_ctx *c, T **p, size_t elem)
     return INMSOM_OK;
 }
 
+// Whole fields between host arrays and the device, collected by add and
+// enqueued together on the context's stream (one kernel packs or unpacks
+// short rows of all of them)
+class Copies {
+  public:
+    explicit Copies(inmsom_ctx *ctx) : c(ctx) {}
+    template <typename T>
+    int add(T *dev, const T *host, int nlev = 1)
+    {
+        if (!host) return set_err(INMSOM_EARG, "NULL host array");
+        f.push_back({(void *)dev, (void *)host, nlev, (int)sizeof(T)});
+        return INMSOM_OK;
+    }
+    int up() { return go(true); }
+    int down() { return go(false); }
+
+  private:
+    inmsom_ctx *c;
+    std::vector<transfer::Field> f;
+    int go(bool to_device)
+    {
+        CK(transfer::rows(c->stage, c->dom, f.data(), (int)f.size(), 0, c->dom.nya() - 1, to_device, c->stream));
+        f.clear();
+        return INMSOM_OK;
+    }
+};
+
+// one field
 template <typename T>
-int h2d(inmsom_ctx *c, T *dev, const T *host)
+int h2d(inmsom_ctx *c, T *dev, const T *host, int nlev = 1)
 {
-    if (!host) return set_err(INMSOM_EARG, "NULL host array");
-    const size_t w = (size_t)c->dom.nxa() * sizeof(T);
-    CK(cudaMemcpy2DAsync(dev + c->dom.xoff, (size_t)c->dom.pitch * sizeof(T), host, w, w,
-                         (size_t)c->dom.nya(), cudaMemcpyHostToDevice, c->stream));
-    return INMSOM_OK;
+    Copies q(c);
+    CKR(q.add(dev, host, nlev));
+    return q.up();
 }
 
 template <typename T>
-int d2h(inmsom_ctx *c, T *host, const T *dev)
+int d2h(inmsom_ctx *c, T *host, const T *dev, int nlev = 1)
 {
-    if (!host) return set_err(INMSOM_EARG, "NULL host array");
-    const size_t w = (size_t)c->dom.nxa() * sizeof(T);
-    CK(cudaMemcpy2DAsync(host, w, dev + c->dom.xoff, (size_t)c->dom.pitch * sizeof(T), w,
-                         (size_t)c->dom.nya(), cudaMemcpyDeviceToHost, c->stream));
-    return INMSOM_OK;
+    Copies q(c);
+    CKR(q.add(const_cast<T *>(dev), host, nlev));
+    return q.down();
 }
 
 int check_bounds(const inmsom_bounds *b);

@@ -1,0 +1,34 @@
+// Copies between the host's contiguous Fortran arrays and the pitched
+// device arrays (see transfer.cu).
+#pragma once
+
+#include <cstddef>
+
+#include "common.cuh"
+
+namespace inmsom {
+namespace transfer {
+
+// one field: device base of its first level (pitched rows, levels pitch *
+// rows apart), host array (bnd_x1:bnd_x2, bnd_y1:bnd_y2, nlev), bytes per
+// element (4 or 8)
+struct Field {
+    void *dev;
+    void *host;
+    int nlev, elem;
+};
+
+// packed device copy of rows on their way; owned by a context, used on one
+// stream, grown on demand
+struct Stage {
+    void *p = nullptr;
+    size_t cap = 0;
+};
+
+// rows r0..r1 (0-based from bnd_y1), whole rows of every level of n fields,
+// to the device (up) or to the host, enqueued on s
+cudaError_t rows(Stage &st, const Dom &d, const Field *f, int n, int r0, int r1, bool up, cudaStream_t s);
+void release(Stage &st);
+
+}  // namespace transfer
+}  // namespace inmsom
