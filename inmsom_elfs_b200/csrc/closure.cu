@@ -28,9 +28,7 @@ namespace {
 
 using namespace inmsom::closure;
 
-constexpr int KIN = 48, HID = 64, NOUT = 2, N3 = 8;
-constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + KIN * HID, OFF_W2 = OFF_B1 + HID, OFF_B2 = OFF_W2 + HID * HID,
-              OFF_W3 = OFF_B2 + HID, OFF_B3 = OFF_W3 + HID * N3, NPARAM = OFF_B3 + N3;
+using namespace inmsom::closure::net;
 constexpr int BOFF_W1 = 0, BOFF_W2 = KIN * HID, BOFF_W3 = BOFF_W2 + HID * HID, NBF = BOFF_W3 + HID * N3;
 static_assert(NPARAM == INMSOM_MLP_NPARAM, "parameter block size");
 constexpr int TILE = 128;     // batch unit of inmsom_mlp_grad (one partial sum set per TILE samples)
@@ -54,23 +52,29 @@ __device__ __forceinline__ void mma16816(float c[4], const uint32_t a[4], const 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// grad[p] = sum over CTAs of partial[c][p] in CTA order (deterministic);
-// grad[NPARAM] = mean squared error
-// 32 parameters per block of 8 warps: warp w sums CTAs w, w+8, ... (each a
-// coalesced 128-byte row piece), then warp 0 adds the 8 sums in order
-__global__ void __launch_bounds__(256) k_mlp_reduce(const float *partial, int ntiles, int batch, float *grad)
+// grad[p] = sum over CTAs of the partial sums of parameter p in CTA order
+// (deterministic); grad[NPARAM] = mean squared error.  32 partial sums per
+// block of RW warps: warp w sums CTAs w, w+RW, ... (each a coalesced 128-byte
+// piece), then warp 0 adds the RW sums in order
+constexpr int RW = 16;
+__global__ void __launch_bounds__(32 * RW) k_mlp_reduce(const float *partial, int ntiles, int batch, float *grad)
 {
-    __shared__ float part[8][32];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, p = 32 * blockIdx.x + l;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ float part[RW][32];
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, i = 32 * blockIdx.x + l;
     float a = 0.f;
-    if (p <= NPARAM)
-        for (int t = w; t < ntiles; t += 8) a += partial[(size_t)t * NPART + p];
+    if (i <= NPARAM) {
+        // added in order, eight loads in flight
+#pragma unroll 8
+        for (int t = w; t < ntiles; t += RW) a += partial[(size_t)t * NPART + i];
+    }
     part[w][l] = a;
     __syncthreads();
-    if (w == 0 && p <= NPARAM) {
+    if (w == 0 && i <= NPARAM) {
         float v = 0.f;
-        for (int k = 0; k < 8; k++) v += part[k][l];
-        grad[p] = p == NPARAM ? v / ((float)batch * NOUT) : v;
+        for (int k = 0; k < RW; k++) v += part[k][l];
+        if (i == NPARAM) grad[i] = v / ((float)batch * NOUT);
+        else grad[partial_param(i)] = v;
     }
 }
 
@@ -78,6 +82,7 @@ __global__ void __launch_bounds__(256) k_mlp_reduce(const float *partial, int nt
 __global__ void k_mlp_adam(float *prm, __nv_bfloat16 *wb, float *m, float *v, const float *grad, int step,
                            float lr, float b1, float b2, float eps)
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= NPARAM) return;
     const bool pad = (p >= OFF_W1 + 45 * HID && p < OFF_B1) || (p >= OFF_W3 && p < OFF_B3 && (p - OFF_W3) % N3 >= NOUT) ||
@@ -501,15 +506,16 @@ int inmsom_mlp_grad(const void *x, const float *targets, const int *idx, int bat
         return fail(INMSOM_EARG, "inmsom_mlp_grad: NULL argument");
     if (batch <= 0 || batch % TILE) return fail(INMSOM_EARG, "inmsom_mlp_grad: batch must be a positive multiple of 128");
     if (ensure_smem()) return INMSOM_ECUDA;
-    // persistent CTAs on the tcgen05 tensor cores, one per SM at most and
-    // at most one per 128 samples (the partial buffer's size)
+    // persistent CTAs on the tcgen05 tensor cores, as many as the SMs hold
+    // and at most one per 128 samples (the partial buffer's size)
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = std::min(batch / TILE, nsm);
+    const int grid = std::min(batch / TILE, inmsom::closure::grad_tc_ctas_per_sm() * nsm);
     if (inmsom::closure::grad_tc(x, targets, idx, batch, params, wbf16, partial, grid, (cudaStream_t)stream))
         return check_launch("inmsom_mlp_grad");
-    k_mlp_reduce<<<(NPARAM + 1 + 31) / 32, 256, 0, (cudaStream_t)stream>>>(partial, grid, batch, grad);
+    (void)inmsom::closure::launch_after(k_mlp_reduce, (NPARAM + 1 + 31) / 32, 32 * RW, 0, (cudaStream_t)stream, partial, grid,
+                                        batch, grad);
     return check_launch("inmsom_mlp_grad reduce");
 }
 
@@ -517,8 +523,8 @@ int inmsom_mlp_adam(float *params, void *wbf16, float *m, float *v, const float 
                     float beta1, float beta2, float eps, void *stream)
 {
     if (!params || !wbf16 || !m || !v || !grad || step < 1) return fail(INMSOM_EARG, "inmsom_mlp_adam: bad argument");
-    k_mlp_adam<<<(NPARAM + 255) / 256, 256, 0, (cudaStream_t)stream>>>(params, (__nv_bfloat16 *)wbf16, m, v, grad,
-                                                                       step, lr, beta1, beta2, eps);
+    (void)inmsom::closure::launch_after(k_mlp_adam, (NPARAM + 63) / 64, 64, 0, (cudaStream_t)stream, params,
+                                        (__nv_bfloat16 *)wbf16, m, v, grad, step, lr, beta1, beta2, eps);
     return check_launch("inmsom_mlp_adam");
 }
 
