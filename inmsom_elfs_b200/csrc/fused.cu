@@ -288,11 +288,16 @@ __device__ __forceinline__ R rcount(int n)
 }
 
 // 1/x by two Newton-Raphson steps r <- r + r*(1 - x*r) (quadratic
-// convergence) from the single-precision reciprocal: about 1 ulp of double
-// for a positive normal x inside the float range, such as a water depth.
+// convergence) from the hardware's approximation of 20 bits: about 1 ulp of
+// double for a positive normal x, such as a water depth.  (From the
+// correctly rounded single-precision reciprocal, with its conversions and
+// its slow-path branch, a substep took 62.5 instead of 59.0 us on 2048 x
+// 1536, 5.15 instead of 4.46 on 256^2, 16.6 instead of 14.2 on a 701 x 487
+// spherical basin; the same results bit for bit.)
 __device__ __forceinline__ double rcp_nr(double x)
 {
-    double r = (double)__frcp_rn((float)x);
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
     double e = fma(-x, r, 1.0);
     r = fma(r, e, r);
     e = fma(-x, r, 1.0);
