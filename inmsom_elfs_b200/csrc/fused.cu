@@ -160,24 +160,22 @@ struct Layout {
                    (GEN ? (int)sizeof(RowCoef) : 0) + (int)sizeof(RowRec));
 };
 
-// ring slots: rows j-1..j+1 in use plus two rows in flight for the plain
-// substep (16 CTAs per SM fit, 20 with FP32 velocities), three in flight
-// where the registers hold the CTAs per SM to 12 (time-mean sums).  What
-// iteration j reads of row j-2 is carried in registers (v at two levels, H
-// + SSH at two levels), which frees its slot an iteration earlier: with one
-// row in flight a quarter of the warps' time went to waiting for rows, the
-// copies' latency being about that of an iteration.  us per substep, before
-// and after: 2048 x 1536 67.3 -> 63.1 (FP32 velocities 55 -> 52), 4096^2
-// FP32 322 -> 309, 256^2 5.4 -> 5.0, 512^2 10.7 -> 9.9
-template <bool GEN, int MODE, bool F32 = false>
-__host__ __device__ constexpr int ring_slots()
-{
-    return (MODE % 3 != 0) ? 6 : 5;
-}
+// ring slots: rows j-1..j+1 in use plus two rows in flight (16 CTAs per SM
+// fit, 20 with FP32 velocities; a third row in flight where registers hold
+// the CTAs per SM to 12, for the time-mean sums, gave nothing: 7.12 against
+// 7.10 ms for a drop-in call's substeps).  What iteration j reads of row j-2
+// is carried in registers (v at two levels, H + SSH at two levels), which
+// frees its slot an iteration earlier: with one row in flight a quarter of
+// the warps' time went to waiting for rows, the copies' latency being about
+// that of an iteration.  us per substep, before and after: 2048 x 1536 67.3
+// -> 63.3 (FP32 velocities 55 -> 52), 4096^2 FP32 322 -> 300, 256^2 5.5 ->
+// 5.2, 512^2 10.7 -> 10.0
+constexpr int RING = 5;
+
 template <bool GEN, int MODE, bool F32 = false>
 constexpr size_t ring_bytes()
 {
-    return (size_t)ring_slots<GEN, MODE, F32>() * (Layout<GEN, F32>::SLOT_B + sizeof(uint64_t));
+    return (size_t)RING * (Layout<GEN, F32>::SLOT_B + sizeof(uint64_t));
 }
 
 // resident CTAs per SM the register budget is cut for: 16 one-warp CTAs
@@ -303,8 +301,15 @@ __device__ __forceinline__ double rcp_nr(double x)
     e = fma(-x, r, 1.0);
     return fma(r, e, r);
 }
-// the FP32 reciprocal, rounded to nearest
-__device__ __forceinline__ float rcp_nr(float x) { return __frcp_rn(x); }
+// the FP32 reciprocal: one Newton step from the hardware's approximation
+// (the correctly rounded function has a slow-path branch: 51.0 instead of
+// 45.3 us per substep on 2048 x 1536)
+__device__ __forceinline__ float rcp_nr(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return fmaf(r, fmaf(-x, r, 1.0f), r);
+}
 
 // state field F of the slot at byte offset o, at the lane's column + dk:
 // FP64, or FP32 velocities widened to FP64
@@ -378,6 +383,7 @@ template <class R>
 struct S2 {
     double sn;               // new SSH of the row (time means only)
     double hs, hsn;          // H + previous SSH and H + new SSH of the row
+    double h, sp;            // FP32 velocities: H and previous SSH instead of their sum
     R vm, vpm;               // v, vp of the row
     R V, Uo;                 // V and U of the row
     R vs;                    // v(k) + v(k+1) of the row
@@ -407,7 +413,6 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
     using L = Layout<GEN, F32>;
     constexpr int ACC = MODE % 3;
     constexpr bool WRITE = MODE / 3 != 0;
-    constexpr int RING = ring_slots<GEN, MODE, F32>();
 
     const int l = threadIdx.x;
     const int g0 = item.x;                     // device column of segment offset 0
@@ -424,8 +429,9 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
 #define AT(o, f, dk) (*reinterpret_cast<const double *>(lane + (o) + L::STAT_OFF + ((f) * SEG + (dk)) * 8))
 #define CF(o, x) (reinterpret_cast<const RowCoef *>(ring + (o) + L::COEF_OFF)->x)
 
+    const int hold = (int)blockIdx.x == p.hold_item ? min(row_lo + p.hold_row, row_hi) : -1;   // test hook
     auto issue = [&](int row, int slot) {
-        if ((int)blockIdx.x == p.hold_item && row == min(row_lo + p.hold_row, row_hi)) return;   // test hook
+        if (row == hold) return;
         issue_row<GEN, F32>(ring + slot * L::SLOT_B, &mbar[slot], tm_src, &p.tm_stat, &p.tm_ssh, &p.tm_rhs, p.rows + row,
                        rec + row, g0, row);
     };
@@ -686,7 +692,11 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
                     hvp = (qc.hs * CF(o_m1, pwv0) + hs * CF(o_m1, pwv1)) * 0.5;
                     hvn = (qc.hsn * CF(o_m1, pwv0) + hsn * CF(o_m1, pwv1)) * 0.5;
                 } else {
-                    hvp = (R)(qc.hs + hs) * R(0.5);
+                    // (the FP32 form sums here: with the sum carried, the
+                    // compiler contracts the v equation's products otherwise
+                    // and the variant's results move by 3e-7)
+                    if constexpr (F32) hvp = (R)((qc.h + qc.sp) + (h0 + AS(o_m1, S_SSHP, 0))) * R(0.5);
+                    else hvp = (R)(qc.hs + hs) * R(0.5);
                     hvn = (R)(qc.hsn + hsn) * R(0.5);
                 }
                 const R gry = qc.Pv - (GX - GXl) - GY - ST * (GEN ? (R)CF(o_m1, pdvt1) : RK(p.d, f_d));
@@ -720,7 +730,12 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
             q.hsn = hsn;
             q.vs = vs;
         }
-        q.hs = hs;
+        if constexpr (F32) {
+            q.h = h0;
+            q.sp = AS(o_m1, S_SSHP, 0);
+        } else {
+            q.hs = hs;
+        }
         q.vm = AV(o_m1, S_V, 0);
         q.vpm = AV(o_m1, S_VP, 0);
         q.V = c.V;
@@ -730,7 +745,10 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
 
         // row j-1 was last read above (what the next iteration needs of it
         // is carried in registers): once every lane is past it, its slot
-        // takes row j-1+RING
+        // takes row j-1+RING.  The proxy fence keeps every lane's reads of
+        // the slot before the copy's writes to it: without it some of them
+        // took place after, with slow loads of time means in between
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (j - 1 + RING <= row_hi) {
             issue(j - 1 + RING, i_m1);
@@ -788,7 +806,6 @@ template <bool GEN, int MODE, bool F32 = false>
 __global__ void __launch_bounds__(NL, min_ctas<GEN, MODE, F32>()) k_substep(const __grid_constant__ Params p)
 {
     using L = Layout<GEN, F32>;
-    constexpr int RING = ring_slots<GEN, MODE, F32>();
     // launched with programmatic stream serialisation: the CTAs may become
     // resident while the previous substep's last CTAs run; nothing global
     // is read or written before that grid has completed
@@ -888,10 +905,10 @@ __global__ void __launch_bounds__(NL, ens_ctas<ANYGEN>())
         const double rs = q.rs_dev[*q.rs_base + st];
         const int4 item = em.items[mi.y];
         if (ANYGEN && em.gen) {
-            uint64_t *mbar = reinterpret_cast<uint64_t *>(ring + ring_slots<true, 3>() * Layout<true>::SLOT_B);
+            uint64_t *mbar = reinterpret_cast<uint64_t *>(ring + RING * Layout<true>::SLOT_B);
             (void)substep_item<true, 3>(q, &q.tm_src, q.dst, rs, item, ring, mbar);
         } else {
-            uint64_t *mbar = reinterpret_cast<uint64_t *>(ring + ring_slots<false, 3>() * Layout<false>::SLOT_B);
+            uint64_t *mbar = reinterpret_cast<uint64_t *>(ring + RING * Layout<false>::SLOT_B);
             (void)substep_item<false, 3>(q, &q.tm_src, q.dst, rs, item, ring, mbar);
         }
         // this item's stores, visible to the bulk copies of later items, then counted
