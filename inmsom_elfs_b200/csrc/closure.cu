@@ -134,14 +134,62 @@ __global__ void k_batch_indices(int *idx, int batch, long long n, unsigned long 
 // the network on 16-cell row segments, the activations of one layer going
 // to the next as MMA fragments in registers.
 constexpr int TCOLS = 64, TROWS = 8, FW = TCOLS + 2, FH = TROWS + 2, NFLD = 5, NTILE = NFLD * FH * FW;
-constexpr int W1S = KIN + 8, W2S = HID + 8;   // padded rows: conflict-free B fragment loads
 static_assert(TROWS == WARPS, "one tile row per warp");
 
+// The network in shared memory as in the parameter block, rows = inputs: the
+// tensor core's B fragments come out of it transposed (ldmatrix.trans), and
+// it is copied 16 bytes at a time.  Rows of W1, W2 padded by 16 bytes: the
+// eight rows of a fragment lie in different banks.
+constexpr int WS = HID + 8;
+struct Weights {
+    alignas(16) __nv_bfloat16 w1[KIN][WS];
+    alignas(16) __nv_bfloat16 w2[HID][WS];
+    alignas(16) __nv_bfloat16 w3[HID][N3];
+    alignas(16) float b1[HID], b2[HID], b3[N3];
+};
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p)
+{
+    return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+// layers 2 and 3 take 2 GELU (gelu2) as their input: their weights are
+// halved here (exact in BF16), so that every product is the network's.
+// Weights that do not start on 16 bytes are read one by one.
+__device__ __forceinline__ void load_weights(Weights &s, const __nv_bfloat16 *wb, const float *prm)
+{
+    constexpr int G = HID / 8, N1 = KIN * G, N2 = HID * G;   // pieces of 8 weights
+    const bool wide = ((uintptr_t)wb & 15) == 0;
+    const __nv_bfloat162 half = __float2bfloat162_rn(0.5f);
+    for (int i = threadIdx.x; i < N1 + N2 + HID; i += blockDim.x) {   // W1, W2, W3 follow each other
+        uint4 v;
+        __nv_bfloat162 *e = reinterpret_cast<__nv_bfloat162 *>(&v);
+        if (wide) {
+            v = reinterpret_cast<const uint4 *>(wb)[i];
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++) e[k] = __halves2bfloat162(wb[8 * i + 2 * k], wb[8 * i + 2 * k + 1]);
+        }
+        if (i >= N1) {
+#pragma unroll
+            for (int k = 0; k < 4; k++) e[k] = __hmul2(e[k], half);
+        }
+        const int j = i < N1 ? i : i - N1;
+        uint4 *dst = i < N1 ? reinterpret_cast<uint4 *>(&s.w1[j / G][8 * (j % G)])
+                     : i < N1 + N2 ? reinterpret_cast<uint4 *>(&s.w2[j / G][8 * (j % G)])
+                                   : reinterpret_cast<uint4 *>(&s.w3[i - N1 - N2][0]);
+        *dst = v;
+    }
+    static_assert(BOFF_W2 == KIN * HID && BOFF_W3 == BOFF_W2 + HID * HID, "consecutive weights");
+    for (int i = threadIdx.x; i < HID; i += blockDim.x) {
+        s.b1[i] = prm[OFF_B1 + i];
+        s.b2[i] = prm[OFF_B2 + i];
+    }
+    if (threadIdx.x < N3) s.b3[threadIdx.x] = prm[OFF_B3 + threadIdx.x];
+}
+
 struct ClSmem {
-    __nv_bfloat16 w1t[HID][W1S];   // W1 transposed, [n][k]
-    __nv_bfloat16 w2t[HID][W2S];
-    __nv_bfloat16 w3t[N3][W2S];
-    float b1[HID], b2[HID], b3[N3];
+    Weights w;
     __nv_bfloat16 tile[NTILE];
     float y[WARPS][16][2];
 };
@@ -152,99 +200,135 @@ __device__ __forceinline__ int feat_off(int k)   // tile offset of feature k, ce
     return f * FH * FW + (q / 3) * FW + (q % 3);
 }
 
-__device__ void stage_tile(__nv_bfloat16 *tile, const inmsom::closure::Args &a, int m0, int n0)
+// the cells m0 .. m0+cols-1 of rows n0 .. n0+TROWS-1 and their ring: a warp
+// per row of a field, lanes along it.  Every load is in flight before the
+// first value is used: one memory latency per tile, not one per row.
+__device__ __forceinline__ void stage_tile(__nv_bfloat16 *tile, const inmsom::closure::Args &a, int m0, int n0, int cols)
 {
-    for (int i = threadIdx.x; i < NTILE; i += blockDim.x) {
-        const int f = i / (FH * FW), rem = i - f * (FH * FW), r = rem / FW, cidx = rem - r * FW;
-        const int m = m0 - 1 + cidx, n = n0 - 1 + r;
-        float v = 0.f;
-        if (m >= a.x1 && m <= a.x2 && n >= a.y1 && n <= a.y2)
-            v = (float)a.fld[f][(long long)(n - a.y1) * a.pitch + (m - a.x1 + a.xoff)];
-        tile[i] = __float2bfloat16((v - a.mean[f]) * a.inv_std[f]);
+    constexpr int RW = (NFLD * FH + WARPS - 1) / WARPS, CW = (FW + 31) / 32;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    double v[RW][CW];
+#pragma unroll
+    for (int i = 0; i < RW; i++) {
+        const int q = w + WARPS * i, f = q / FH, n = n0 - 1 + q - f * FH;
+        const bool in = q < NFLD * FH && n >= a.y1 && n <= a.y2;
+        const double *row = in ? a.fld[f] + (long long)(n - a.y1) * a.pitch + (a.xoff - a.x1) : nullptr;
+#pragma unroll
+        for (int j = 0; j < CW; j++) {
+            const int c = l + 32 * j, m = m0 - 1 + c;
+            v[i][j] = in && c < cols + 2 && m >= a.x1 && m <= a.x2 ? row[m] : 0.0;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < RW; i++) {
+        const int q = w + WARPS * i;
+        if (q >= NFLD * FH) break;
+        const float mean = a.mean[q / FH], inv = a.inv_std[q / FH];
+#pragma unroll
+        for (int j = 0; j < CW; j++)
+            if (l + 32 * j < FW) tile[q * FW + l + 32 * j] = __float2bfloat16(((float)v[i][j] - mean) * inv);
     }
 }
 
-__device__ __forceinline__ uint32_t lds32(const __nv_bfloat16 *p) { return *reinterpret_cast<const uint32_t *>(p); }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi)
 {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&v);
 }
 
-// y (outputs 0, 1 of cells g and g+8 in o[0..3] of lanes t == 0) of the
-// 16 cells whose layer-1 A fragments are a1.  The hidden activations are
-// kept as 2 GELU (gelu2) and s.w2t, s.w3t hold the halved weights: the same
-// products, one multiplication fewer per activation.
-template <class S>
-__device__ __forceinline__ void mlp16(const S &s, const uint32_t a1[3][4], float o[4])
+// four 8 x 8 blocks of B, transposed: the fragments of two MMAs
+__device__ __forceinline__ void ldsm4t(uint32_t r[4], const void *p)
 {
-    const int l = threadIdx.x & 31, g = l >> 2, t = l & 3;
-    float acc[8][4];
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(smem_addr(p)));
+}
+
+// c[nt] += A[kb] B: KB blocks of 16 inputs, 64 outputs
+template <int KB>
+__device__ __forceinline__ void layer(float acc[8][4], const uint32_t (*a)[4], const __nv_bfloat16 (*w)[WS])
+{
+    const int l = threadIdx.x & 31;
+    const __nv_bfloat16 *p = &w[(l & 7) + 8 * ((l >> 3) & 1)][8 * (l >> 4)];
 #pragma unroll
-    for (int nt = 0; nt < 8; nt++) {
-        acc[nt][0] = acc[nt][2] = s.b1[8 * nt + 2 * t];
-        acc[nt][1] = acc[nt][3] = s.b1[8 * nt + 2 * t + 1];
-    }
+    for (int kb = 0; kb < KB; kb++)
 #pragma unroll
-    for (int kb = 0; kb < 3; kb++)
-#pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
-            const uint32_t b[2] = {lds32(&s.w1t[8 * nt + g][16 * kb + 2 * t]), lds32(&s.w1t[8 * nt + g][16 * kb + 2 * t + 8])};
-            mma16816(acc[nt], a1[kb], b);
+        for (int nt = 0; nt < 8; nt += 2) {
+            uint32_t b[4];
+            ldsm4t(b, p + 16 * kb * WS + 8 * nt);
+            mma16816(acc[nt], a[kb], b);
+            mma16816(acc[nt + 1], a[kb], b + 2);
         }
-    uint32_t a2[4][4];
-#pragma unroll
-    for (int kb = 0; kb < 4; kb++) {
-        a2[kb][0] = pack2(gelu2(acc[2 * kb][0]), gelu2(acc[2 * kb][1]));
-        a2[kb][1] = pack2(gelu2(acc[2 * kb][2]), gelu2(acc[2 * kb][3]));
-        a2[kb][2] = pack2(gelu2(acc[2 * kb + 1][0]), gelu2(acc[2 * kb + 1][1]));
-        a2[kb][3] = pack2(gelu2(acc[2 * kb + 1][2]), gelu2(acc[2 * kb + 1][3]));
-    }
-#pragma unroll
-    for (int nt = 0; nt < 8; nt++) {
-        acc[nt][0] = acc[nt][2] = s.b2[8 * nt + 2 * t];
-        acc[nt][1] = acc[nt][3] = s.b2[8 * nt + 2 * t + 1];
-    }
+}
+
+// 2 GELU of an accumulator block as the next layer's A fragments
+__device__ __forceinline__ void activate(uint32_t a2[4][4], const float acc[8][4])
+{
 #pragma unroll
     for (int kb = 0; kb < 4; kb++)
 #pragma unroll
-        for (int nt = 0; nt < 8; nt++) {
-            const uint32_t b[2] = {lds32(&s.w2t[8 * nt + g][16 * kb + 2 * t]), lds32(&s.w2t[8 * nt + g][16 * kb + 2 * t + 8])};
-            mma16816(acc[nt], a2[kb], b);
+        for (int q = 0; q < 4; q++) {
+            float x = acc[2 * kb + (q >> 1)][2 * (q & 1)], y = acc[2 * kb + (q >> 1)][2 * (q & 1) + 1];
+            gelu2_pair(x, y);
+            a2[kb][q] = pack2(x, y);
         }
+}
+
+__device__ __forceinline__ void bias(float acc[8][4], const float *b)
+{
+    const int t = threadIdx.x & 3;
 #pragma unroll
-    for (int kb = 0; kb < 4; kb++) {
-        a2[kb][0] = pack2(gelu2(acc[2 * kb][0]), gelu2(acc[2 * kb][1]));
-        a2[kb][1] = pack2(gelu2(acc[2 * kb][2]), gelu2(acc[2 * kb][3]));
-        a2[kb][2] = pack2(gelu2(acc[2 * kb + 1][0]), gelu2(acc[2 * kb + 1][1]));
-        a2[kb][3] = pack2(gelu2(acc[2 * kb + 1][2]), gelu2(acc[2 * kb + 1][3]));
-    }
-    o[0] = o[2] = s.b3[2 * t];
-    o[1] = o[3] = s.b3[2 * t + 1];
-#pragma unroll
-    for (int kb = 0; kb < 4; kb++) {
-        const uint32_t b[2] = {lds32(&s.w3t[g][16 * kb + 2 * t]), lds32(&s.w3t[g][16 * kb + 2 * t + 8])};
-        mma16816(o, a2[kb], b);
+    for (int nt = 0; nt < 8; nt++) {
+        const float2 v = *reinterpret_cast<const float2 *>(&b[8 * nt + 2 * t]);
+        acc[nt][0] = acc[nt][2] = v.x;
+        acc[nt][1] = acc[nt][3] = v.y;
     }
 }
 
-// Persistent over tiles: out[c] = base[c] + MLP(features)_c * out_scale[c] * fac[c]
+// y (outputs 0, 1 of cells g and g+8 in o[0..3] of lanes t == 0) of the
+// 16 cells whose layer-1 A fragments are a1.  The hidden activations are
+// kept as 2 GELU (gelu2), the weights of layers 2 and 3 halved: the same
+// products, one multiplication fewer per activation.
+__device__ __forceinline__ void mlp16(const Weights &s, const uint32_t a1[3][4], float o[4])
+{
+    const int l = threadIdx.x & 31, t = l & 3;
+    float acc[8][4];
+    uint32_t a2[4][4];
+    bias(acc, s.b1);
+    layer<3>(acc, a1, s.w1);
+    activate(a2, acc);
+    bias(acc, s.b2);
+    layer<4>(acc, a2, s.w2);
+    activate(a2, acc);
+    o[0] = o[2] = s.b3[2 * t];
+    o[1] = o[3] = s.b3[2 * t + 1];
+#pragma unroll
+    for (int kb = 0; kb < 4; kb += 2) {
+        uint32_t b[4];
+        ldsm4t(b, &s.w3[16 * kb + l][0]);
+        mma16816(o, a2[kb], b);
+        mma16816(o, a2[kb + 1], b + 2);
+    }
+}
+
+__host__ __device__ inline long long apply_units(const inmsom::closure::Args &a)
+{
+    return (long long)((a.mx1 - a.mx0 + 16) / 16) * ((a.ny1 - a.ny0 + TROWS) / TROWS);
+}
+
+// out[c] = base[c] + MLP(features)_c * out_scale[c] * fac[c].  Bound by the
+// instructions issued and the matrix and tanh pipes together (16.6 M warp
+// instructions on 512 x 512 cells with B fragments by 4-byte loads and GELU
+// value by value, 11.8 M now; 46 % of the issue slots).  Work is cut in units
+// of TROWS rows x 16 columns; every CTA has an equal share of consecutive
+// units (whole tiles of 64 columns left 512 x 512 cells at 4 or 8 units per
+// CTA where 7 are enough) and stages up to TCOLS columns of them at a time.
+// An evaluation between substeps on 512 x 512 cells: 38 us before, 32 with
+// the fragments and GELU above, 29 with the units and a tile's loads at once.
 __global__ void __launch_bounds__(WARPS * 32, 2) k_closure_apply(const __grid_constant__ inmsom::closure::Args a)
 {
     __shared__ __align__(16) ClSmem s;
-    const __nv_bfloat16 *wb = (const __nv_bfloat16 *)a.wb;
-    for (int i = threadIdx.x; i < KIN * HID; i += blockDim.x) s.w1t[i % HID][i / HID] = wb[BOFF_W1 + i];
-    // layers 2 and 3 take 2 GELU (gelu2) as their input: their weights are
-    // halved here (exact in BF16), so that every product is the network's
-    for (int i = threadIdx.x; i < HID * HID; i += blockDim.x)
-        s.w2t[i % HID][i / HID] = __float2bfloat16(0.5f * __bfloat162float(wb[BOFF_W2 + i]));
-    for (int i = threadIdx.x; i < HID * N3; i += blockDim.x)
-        s.w3t[i % N3][i / N3] = __float2bfloat16(0.5f * __bfloat162float(wb[BOFF_W3 + i]));
-    for (int i = threadIdx.x; i < HID; i += blockDim.x) {
-        s.b1[i] = a.prm[OFF_B1 + i];
-        s.b2[i] = a.prm[OFF_B2 + i];
-    }
-    if (threadIdx.x < N3) s.b3[threadIdx.x] = a.prm[OFF_B3 + threadIdx.x];
+    load_weights(s.w, (const __nv_bfloat16 *)a.wb, a.prm);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, g = l >> 2, t = l & 3;
     // this lane's 12 feature offsets of the layer-1 A fragments (k >= 45: zero)
     int koff[3][4];
@@ -255,17 +339,20 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_closure_apply(const __grid_co
             const int k = 16 * kb + 2 * t + (q & 1) + 8 * (q >> 1);
             koff[kb][q] = k < 45 ? feat_off(k) : -1;
         }
-    const int nx = a.mx1 - a.mx0 + 1, ny = a.ny1 - a.ny0 + 1;
-    const int ntx = (nx + TCOLS - 1) / TCOLS, nty = (ny + TROWS - 1) / TROWS;
+    const long long units = apply_units(a);
+    const int upr = (a.mx1 - a.mx0 + 16) / 16;   // units per row of them
     const __nv_bfloat16 zero = __float2bfloat16(0.f);
-    for (int tix = blockIdx.x; tix < ntx * nty; tix += gridDim.x) {
-        const int m0 = a.mx0 + (tix % ntx) * TCOLS, n0 = a.ny0 + (tix / ntx) * TROWS;
+    const long long u1 = units * (blockIdx.x + 1) / gridDim.x;
+    for (long long u = units * blockIdx.x / gridDim.x; u < u1;) {
+        const int q = (int)(u % upr), cols = 16 * (int)min(min(u1 - u, (long long)(upr - q)), (long long)(TCOLS / 16));
+        const int m0 = a.mx0 + 16 * q, n0 = a.ny0 + (int)(u / upr) * TROWS;
+        u += cols / 16;
         __syncthreads();   // the previous tile's reads are done (and the weights are in)
-        stage_tile(s.tile, a, m0, n0);
+        stage_tile(s.tile, a, m0, n0, cols);
         __syncthreads();
         const int n = n0 + w;
         if (n > a.ny1) continue;
-        for (int c0 = 0; c0 < TCOLS && m0 + c0 <= a.mx1; c0 += 16) {
+        for (int c0 = 0; c0 < cols; c0 += 16) {
             uint32_t a1[3][4];
             const int base_g = w * FW + c0 + g, base_h = base_g + 8;   // cells g, g+8 at ring offset
 #pragma unroll
@@ -279,7 +366,7 @@ __global__ void __launch_bounds__(WARPS * 32, 2) k_closure_apply(const __grid_co
                     a1[kb][2 * h + 1] = pack_raw(xh0, xh1);
                 }
             float o[4];
-            mlp16(s, a1, o);
+            mlp16(s.w, a1, o);
             if (t == 0) {
                 s.y[w][g][0] = o[0];
                 s.y[w][g][1] = o[1];
@@ -311,7 +398,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_closure_features(const __grid_co
     for (int tix = blockIdx.x; tix < ntx * nty; tix += gridDim.x) {
         const int m0 = a.mx0 + (tix % ntx) * TCOLS, n0 = a.ny0 + (tix / ntx) * TROWS;
         __syncthreads();
-        stage_tile(tile, a, m0, n0);
+        stage_tile(tile, a, m0, n0, TCOLS);
         __syncthreads();
         const int n = n0 + w;
         if (n > a.ny1) continue;
@@ -345,12 +432,7 @@ __global__ void k_closure_factors(inmsom::closure::Args a, const float *lcu, con
 // Here: the network of k_closure_apply on rows of features, 64 samples per
 // tile, one warp per 16.
 constexpr int GT = 64, GW = 4;            // samples per tile, warps per CTA
-constexpr int XS = KIN + 8, HS = HID + 8;  // padded row strides (16-byte rows, conflict-free)
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p)
-{
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
+constexpr int XS = KIN + 8;               // padded row stride (16-byte rows, conflict-free)
 
 __device__ __forceinline__ void ldsm4(uint32_t r[4], const void *p)
 {
@@ -362,10 +444,7 @@ __device__ __forceinline__ void ldsm4(uint32_t r[4], const void *p)
 // y[n][0..1] = MLP(x[n]) for n < count: the network of k_closure_apply
 // (mlp16) on feature rows, 64 per tile, one warp per 16
 struct FSmem {
-    alignas(16) __nv_bfloat16 w1t[HID][XS];
-    alignas(16) __nv_bfloat16 w2t[HID][HS];
-    alignas(16) __nv_bfloat16 w3t[16][HS];
-    float b1[HID], b2[HID], b3[N3];
+    Weights w;
     alignas(16) __nv_bfloat16 x[GT][XS];
 };
 
@@ -374,20 +453,7 @@ __global__ void __launch_bounds__(GW * 32) k_mlp_forward(const __nv_bfloat16 *x,
 {
     __shared__ FSmem s;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, g = l >> 2, t = l & 3;
-    for (int i = threadIdx.x; i < KIN * HID; i += blockDim.x) s.w1t[i % HID][i / HID] = wb[BOFF_W1 + i];
-    // layers 2 and 3 take 2 GELU (mlp16's gelu2): their weights halved (exact)
-    for (int i = threadIdx.x; i < HID * HID; i += blockDim.x)
-        s.w2t[i % HID][i / HID] = __float2bfloat16(0.5f * __bfloat162float(wb[BOFF_W2 + i]));
-    for (int i = threadIdx.x; i < 16 * HS; i += blockDim.x) {
-        const int o = i / HS, c = i % HS;
-        s.w3t[o][c] = o < N3 && c < HID ? __float2bfloat16(0.5f * __bfloat162float(wb[BOFF_W3 + c * N3 + o]))
-                                        : __float2bfloat16(0.f);
-    }
-    for (int i = threadIdx.x; i < HID; i += blockDim.x) {
-        s.b1[i] = prm[OFF_B1 + i];
-        s.b2[i] = prm[OFF_B2 + i];
-    }
-    if (threadIdx.x < N3) s.b3[threadIdx.x] = prm[OFF_B3 + threadIdx.x];
+    load_weights(s.w, wb, prm);
     const int m0 = 16 * w;
     const long long ntiles = (count + GT - 1) / GT;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -404,7 +470,7 @@ __global__ void __launch_bounds__(GW * 32) k_mlp_forward(const __nv_bfloat16 *x,
 #pragma unroll
         for (int kb = 0; kb < 3; kb++) ldsm4(a1[kb], &s.x[m0 + (l & 7) + 8 * ((l >> 3) & 1)][16 * kb + 8 * (l >> 4)]);
         float o[4];
-        mlp16(s, a1, o);
+        mlp16(s.w, a1, o);
         if (t == 0) {
             const long long r0 = tile * GT + m0 + g, r1 = r0 + 8;
             if (r0 < count) {
@@ -449,9 +515,8 @@ namespace closure {
 
 int apply(const Args &a, int nsm, cudaStream_t s)
 {
-    const int nx = a.mx1 - a.mx0 + 1, ny = a.ny1 - a.ny0 + 1;
-    const int tiles = ((nx + TCOLS - 1) / TCOLS) * ((ny + TROWS - 1) / TROWS);
-    const int grid = tiles < 2 * nsm ? tiles : 2 * nsm;
+    const long long units = apply_units(a);
+    const int grid = (int)(units < 2 * nsm ? units : 2 * nsm);
     k_closure_apply<<<grid, WARPS * 32, 0, s>>>(a);
     return check_launch("closure apply");
 }

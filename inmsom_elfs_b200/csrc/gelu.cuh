@@ -35,6 +35,19 @@ __device__ __forceinline__ float gelu2(float x)
     return fmaf(x, tanh_hw(x * fmaf(GELU_C1, x * x, GELU_C0)), x);
 }
 
+// gelu2 of two values at once, in the two-wide FP32 instructions (each half
+// rounds as the single one does)
+__device__ __forceinline__ void gelu2_pair(float &x, float &y)
+{
+    asm("{\n\t.reg .b64 v, q, c0, c1;\n\t.reg .f32 a, b;\n\t"
+        "mov.b64 v, {%0, %1};\n\tmov.b64 c0, {%2, %2};\n\tmov.b64 c1, {%3, %3};\n\t"
+        "mul.rn.f32x2 q, v, v;\n\tfma.rn.f32x2 q, c1, q, c0;\n\tmul.rn.f32x2 q, v, q;\n\t"
+        "mov.b64 {a, b}, q;\n\ttanh.approx.f32 a, a;\n\ttanh.approx.f32 b, b;\n\tmov.b64 q, {a, b};\n\t"
+        "fma.rn.f32x2 v, v, q, v;\n\tmov.b64 {%0, %1}, v;\n\t}"
+        : "+f"(x), "+f"(y)
+        : "f"(GELU_C0), "f"(GELU_C1));
+}
+
 __device__ __forceinline__ float gelu_d(float x)
 {
     const float x2 = x * x, t = tanh_hw(x * fmaf(GELU_C1, x2, GELU_C0));

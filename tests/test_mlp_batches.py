@@ -48,3 +48,24 @@ def test_gradient_matches_oracle(gpu, tiles):
     cuts = (o.OFF_W1, o.OFF_B1, o.OFF_W2, o.OFF_B2, o.OFF_W3, o.OFF_B3, o.NPARAM)
     for a, b in zip(cuts[:-1], cuts[1:]):
         assert np.abs(got[a:b] - want[a:b]).max() <= 2e-2 * np.abs(want[a:b]).max(), (a, b)
+
+
+@pytest.mark.parametrize("rows", [1, 15, 64, 65, 4099])
+def test_forward_wherever_the_weights_start(gpu, rows):
+    """Weights read 16 bytes at a time where they start on 16 bytes, one by
+    one elsewhere: the same values, and the oracle's within the 2e-3 of the
+    hardware tanh (2^-11) and the BF16 activations."""
+    import torch
+    from inmsom_elfs_b200 import _lib
+    from inmsom_elfs_b200.mlp import MLP
+    every = _data(33)[0]
+    x = every[:rows].contiguous()
+    net = MLP(seed=rows)
+    want = net.forward(x).cpu().numpy()
+    y, _ = mlp_oracle.forward(net.host_params(), every.float().cpu().numpy(), emulate=True)
+    assert np.abs(want - y[:rows]).max() <= 2e-3 * np.abs(y).max()
+    room = torch.empty(_lib.MLP_NBF16 + 8, dtype=torch.bfloat16, device="cuda")
+    for off in (1, 4, 7):
+        net2 = MLP(net.host_params())
+        net2.wbf16 = room[off:off + _lib.MLP_NBF16].copy_(net.wbf16)
+        assert np.array_equal(net2.forward(x).cpu().numpy(), want), off
