@@ -24,14 +24,14 @@
 // branch-free (masked selects, predicated stores) except for warp-wide skips
 // of rows without ocean.
 //
-// Input rows j-1..j+1 sit in a ring of RING shared-memory slots.  A slot
+// Input rows j-1..j+1 sit in a ring of 4 or 5 (RS) shared-memory slots.  A slot
 // holds a 36-column segment of the six state fields and of the static
 // fields (rest depth, forcing; in the general variant also viscosity, drag
 // and water flux), brought by two 3-D tiled TMA loads from field-blocked
 // arrays (cp.async.bulk.tensor, each copy for one CTA), plus the strip's T-mask bits
 // and Coriolis factor of the row (and, in the general variant, its metric
 // coefficients) by 1-D bulk copies.  One elected lane refills the slot of row
-// j-1 with row j-1+RING once every lane is past it; the few values of it that
+// j-1 with row j-1+RS once every lane is past it; the few values of it that
 // the next iteration reads are carried in registers.  Every wait is bounded: on timeout the CTA sets a status bit,
 // drains its own copies (bounded) and returns.
 //
@@ -160,39 +160,48 @@ struct Layout {
                    (GEN ? (int)sizeof(RowCoef) : 0) + (int)sizeof(RowRec));
 };
 
-// ring slots: rows j-1..j+1 in use plus two rows in flight (16 CTAs per SM
-// fit, 20 with FP32 velocities; a third row in flight where registers hold
-// the CTAs per SM to 12, for the time-mean sums, gave nothing: 7.12 against
-// 7.10 ms for a drop-in call's substeps).  What iteration j reads of row j-2
-// is carried in registers (v at two levels, H + SSH at two levels), which
-// frees its slot an iteration earlier: with one row in flight a quarter of
-// the warps' time went to waiting for rows, the copies' latency being about
-// that of an iteration.  us per substep, before and after: 2048 x 1536 67.3
-// -> 63.3 (FP32 velocities 55 -> 52), 4096^2 FP32 322 -> 300, 256^2 5.5 ->
-// 5.2, 512^2 10.7 -> 10.0
-constexpr int RING = 5;
+// Ring slots: rows j-1..j+1 in use plus the rows in flight.  What iteration j
+// reads of row j-2 is carried in registers (v at two levels, H + SSH at two
+// levels), which frees its slot an iteration earlier: with that slot in
+// use and one row in flight a quarter of the warps' time went to waiting for
+// rows (us per substep, before and after: 2048 x 1536 67.3 -> 63.3, FP32
+// velocities 55 -> 52, 4096^2 FP32 322 -> 300).
+// RING: two rows in flight (16 CTAs per SM fit, 20 with FP32 velocities; a
+// third row where registers hold the CTAs to 12, for the time-mean sums,
+// gave nothing: 7.12 against 7.10 ms for a drop-in call's substeps).
+// SHORT_RING: one row in flight.  Better for the plain FP64 substep of a
+// basin alone whose items make few waves (build_table has the rule): there
+// all CTAs start together and the second row's copies only queue in front of
+// the rows needed next.  us per substep with 5 and 4 slots: 512^2 9.2, 8.6;
+// 1024^2 31.1, 28.4; 700 x 500 9.6, 8.8; 2048 x 1536 58.9, 57.6; general
+// variant 701 x 487 14.1, 13.4 (12 CTAs per SM fit instead of 11), 1024 x 768
+// 32.4, 30.4.  Slower with FP32 velocities (45.3, 46.2) and for the members
+// of an ensemble, whose items are long (56.2, 57.2).
+constexpr int RING = 5, SHORT_RING = 4;
 
 template <bool GEN, int MODE, bool F32 = false>
-constexpr size_t ring_bytes()
+constexpr size_t ring_bytes(int slots = RING)
 {
-    return (size_t)RING * (Layout<GEN, F32>::SLOT_B + sizeof(uint64_t));
+    return (size_t)slots * (Layout<GEN, F32>::SLOT_B + sizeof(uint64_t));
 }
 
 // resident CTAs per SM the register budget is cut for: 16 one-warp CTAs
 // (4 warps per SM sub-partition, 128 registers) for the plain substep, 20
 // (5 warps per sub-partition, 96 registers) for its FP32-velocity form with
 // FP32 momentum arithmetic, 12 where the time-mean sums need more registers,
-// 11 for the general variant, and never more than the shared memory holds
-// (228 KB per SM, 1 KB of it reserved per CTA): 16 for the FP64 uniform ring
-// of 5 slots, 20 for the FP32 one, 11 for the general one.  (A 6-slot ring holds 13 uniform CTAs: 6 % slower on the
-// 2048 x 1536 basin; 128 bytes of alignment slack per CTA leave room for 15:
-// 2 % slower; reading the forcing from global memory instead of the ring
-// exposes the load latency: 5 % slower.)
+// 12 for the general variant too, and never more than the shared memory
+// holds (228 KB per SM, 1 KB of it reserved per CTA): 16 for the FP64 uniform
+// ring of 5 slots, 20 for the FP32 one, 11 for the general one (13 with 4
+// slots).  (A 6-slot ring holds 13 uniform CTAs: 6 % slower on the 2048 x
+// 1536 basin; 128 bytes of alignment slack per CTA leave room for 15: 2 %
+// slower; 20 CTAs of 4 slots at 96 registers with a few bytes spilled: 8 %
+// slower; reading the forcing from global memory instead of the ring exposes
+// the load latency: 5 % slower.)
 template <bool GEN, int MODE, bool F32 = false>
 constexpr int min_ctas()
 {
-    constexpr int by_smem = (int)(233472 / (ring_bytes<GEN, MODE, F32>() + 1024));
-    constexpr int want = GEN ? 11 : (MODE % 3 ? 12 : (F32 ? 20 : 16));
+    constexpr int by_smem = (int)(233472 / (ring_bytes<GEN, MODE, F32>(MODE == 3 && !F32 ? SHORT_RING : RING) + 1024));
+    constexpr int want = GEN ? 12 : (MODE % 3 ? 12 : (F32 ? 20 : 16));
     return by_smem < want ? by_smem : want;
 }
 static_assert(NSET * SEG * 8 <= 1792, "state segment overlaps the static segment");
@@ -406,7 +415,7 @@ using On = std::integral_constant<bool, B>;
 // gave up (FLAG_TIMEOUT is set).
 // MODE = acc + 3*write: acc 0 none, 1 first substep (write), 2 accumulate;
 // write 1 stores the new state
-template <bool GEN, int MODE, bool F32 = false>
+template <bool GEN, int MODE, bool F32 = false, int RS = RING>
 __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap *tm_src, double *const *dst,
                                              const double rs, const int4 item, unsigned char *ring, uint64_t *mbar)
 {
@@ -441,12 +450,12 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
     };
 
     if (l == 0) {
-        for (int s = 0; s < RING; s++) mbar_init(&mbar[s], 1);
+        for (int s = 0; s < RS; s++) mbar_init(&mbar[s], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
     int issued = row_lo - 1;
-    for (int t = 0; t < RING && row_lo + t <= row_hi; t++) issue(row_lo + t, t), issued = row_lo + t;
+    for (int t = 0; t < RS && row_lo + t <= row_hi; t++) issue(row_lo + t, t), issued = row_lo + t;
 
     const bool out = l >= 1 && l <= NL - 2 && k >= p.c_first && k <= p.c_last;
     const double gam = p.gam, two_ti = p.two_ti;
@@ -637,7 +646,7 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
         // test (without waiting) whether row j+2 has arrived, so that the
         // next iteration's branch on it does not wait for the test
         {
-            const int ns = i_p1 == RING - 1 ? 0 : i_p1 + 1;
+            const int ns = i_p1 == RS - 1 ? 0 : i_p1 + 1;
             ready = mbar_test(&mbar[ns], ph ^ (ns == 0 ? 1u : 0u));
         }
 
@@ -745,18 +754,18 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
 
         // row j-1 was last read above (what the next iteration needs of it
         // is carried in registers): once every lane is past it, its slot
-        // takes row j-1+RING.  The proxy fence keeps every lane's reads of
+        // takes row j-1+RS.  The proxy fence keeps every lane's reads of
         // the slot before the copy's writes to it: without it some of them
         // took place after, with slow loads of time means in between
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (j - 1 + RING <= row_hi) {
-            issue(j - 1 + RING, i_m1);
-            issued = j - 1 + RING;
+        if (j - 1 + RS <= row_hi) {
+            issue(j - 1 + RS, i_m1);
+            issued = j - 1 + RS;
         }
         i_m1 = i_0;
         i_0 = i_p1;
-        i_p1 = i_p1 == RING - 1 ? 0 : i_p1 + 1;
+        i_p1 = i_p1 == RS - 1 ? 0 : i_p1 + 1;
         ph ^= i_p1 == 0 ? 1u : 0u;
         gi += p.pitch;
     };
@@ -784,7 +793,7 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
             atomicOr(p.flags, FLAG_TIMEOUT);
             // drain this CTA's copies still in flight (bounded) before exiting
             for (int row = waited + 1; row <= issued; row++)
-                (void)mbar_wait(&mbar[(row - row_lo) % RING], (uint32_t)(((row - row_lo) / RING) & 1),
+                (void)mbar_wait(&mbar[(row - row_lo) % RS], (uint32_t)(((row - row_lo) / RS) & 1),
                                 p.wait_limit);
         }
         return false;
@@ -792,7 +801,7 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
     // every copy issued was waited for: the barriers can be retired
     __syncwarp();
     if (l == 0)
-        for (int t = 0; t < RING; t++) mbar_inval(&mbar[t]);
+        for (int t = 0; t < RS; t++) mbar_inval(&mbar[t]);
     __syncwarp();
     return true;
 #undef AS
@@ -802,7 +811,7 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
 #undef CF
 }
 
-template <bool GEN, int MODE, bool F32 = false>
+template <bool GEN, int MODE, bool F32 = false, int RS = RING>
 __global__ void __launch_bounds__(NL, min_ctas<GEN, MODE, F32>()) k_substep(const __grid_constant__ Params p)
 {
     using L = Layout<GEN, F32>;
@@ -818,9 +827,9 @@ __global__ void __launch_bounds__(NL, min_ctas<GEN, MODE, F32>()) k_substep(cons
         if (threadIdx.x == 0) atomicOr(p.flags, FLAG_SMEM);
         return;
     }
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(ring + RING * L::SLOT_B);
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(ring + RS * L::SLOT_B);
     const double rs = p.rs_dev ? p.rs_dev[*p.rs_base + p.rs_k] : p.rhs_scale;
-    (void)substep_item<GEN, MODE, F32>(p, &p.tm_src, p.dst, rs, p.items[p.turn ? gridDim.x - 1 - blockIdx.x : blockIdx.x], ring, mbar);
+    (void)substep_item<GEN, MODE, F32, RS>(p, &p.tm_src, p.dst, rs, p.items[p.turn ? gridDim.x - 1 - blockIdx.x : blockIdx.x], ring, mbar);
 }
 
 // ---------------------------------------------------------------------
@@ -1084,20 +1093,27 @@ int set_io(const Plan &p, Params &q, double *const src[NSET], double *const dst[
 // a substep launch that may start while the previous one drains (the
 // kernel waits for it with griddepcontrol.wait before touching memory):
 // 2 % on the time-mean substeps of a drop-in call, none under graph replay
-template <bool GEN, int MODE, bool F32 = false>
+template <bool GEN, int MODE, bool F32 = false, int RS = RING>
 void launch_substep(int grid, const Params &q, cudaStream_t s)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(NL);
-    cfg.dynamicSmemBytes = ring_bytes<GEN, MODE, F32>();
+    cfg.dynamicSmemBytes = ring_bytes<GEN, MODE, F32>(RS);
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    (void)cudaLaunchKernelEx(&cfg, k_substep<GEN, MODE, F32>, q);   // errors: cudaGetLastError
+    (void)cudaLaunchKernelEx(&cfg, k_substep<GEN, MODE, F32, RS>, q);   // errors: cudaGetLastError
+}
+
+template <bool GEN>
+void launch_plain(int ring, int grid, const Params &q, cudaStream_t s)
+{
+    if (ring == SHORT_RING) launch_substep<GEN, 3, false, SHORT_RING>(grid, q, s);
+    else launch_substep<GEN, 3>(grid, q, s);
 }
 
 template <bool GEN, int MODE>
@@ -1107,7 +1123,8 @@ void launch_t(const Plan &p, const Params &q, cudaStream_t s)
     Params r = q;
     r.items = p.items[v];
     r.turn = q.turn && p.turn[v];
-    launch_substep<GEN, MODE>(p.nitems[v], r, s);
+    if constexpr (MODE == 3) launch_plain<GEN>(p.ring[v], p.nitems[v], r, s);
+    else launch_substep<GEN, MODE>(p.nitems[v], r, s);
 }
 
 // mode = acc + 3*write (acc: 0 none, 1 write, 2 accumulate)
@@ -1163,6 +1180,10 @@ int set_smem()
 {
     return set_smem1<false, 2>() | set_smem1<false, 3>() | set_smem1<false, 4>() | set_smem1<false, 5>() |
            set_smem1<true, 2>() | set_smem1<true, 3>() | set_smem1<true, 4>() | set_smem1<true, 5>() |
+           (cudaFuncSetAttribute(k_substep<false, 3, false, SHORT_RING>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)ring_bytes<false, 3>(SHORT_RING)) != cudaSuccess) |
+           (cudaFuncSetAttribute(k_substep<true, 3, false, SHORT_RING>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)ring_bytes<true, 3>(SHORT_RING)) != cudaSuccess) |
            (cudaFuncSetAttribute(k_substep<false, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)ring_bytes<false, 3, true>()) != cudaSuccess);
 }
@@ -1315,10 +1336,11 @@ std::vector<int4> partition(const Plan &p, const Dom &d, int slots, int rows_per
 }
 
 constexpr double L2_BYTES = 126e6;
+constexpr int SHORT_WAVES = 4;
 
 // Replaces table v.  On failure the plan keeps its previous table (a
 // launch never sees a count without its items).
-int upload_items(Plan &p, int v, const std::vector<int4> &items, cudaStream_t s)
+int upload_items(Plan &p, int v, const std::vector<int4> &items, int slots, int ring, cudaStream_t s)
 {
     int4 *t = nullptr;
     if (cudaMalloc(&t, items.size() * sizeof(int4)) != cudaSuccess) return 1;
@@ -1332,18 +1354,34 @@ int upload_items(Plan &p, int v, const std::vector<int4> &items, cudaStream_t s)
     cudaFree(p.items[v]);
     p.items[v] = t;
     p.nitems[v] = (int)items.size();
+    p.ring[v] = ring;
     // Alternate substeps run through the table from its two ends, so that
     // a substep starts with the rows the last one wrote at its end, while
     // they are in L2: where the items are several waves and one wave's rows
     // fit it (2048 x 1536: 63.3 -> 62.5 us per substep, FP32 velocities 52.1
     // -> 51.1, the drop-in call's 100 substeps 7.71 -> 7.49 ms; with one wave
     // or past L2 it lost 1-6 %: 512^2 10.0 -> 10.7, 4096^2 FP32 300 -> 302 us).
-    const int slots = p.nsm * p.occ[v];
     double rows = 0.0;
     for (const int4 &it : items) rows += it.z - it.y;
     const double cell = v == TABLE_F32 ? 80.0 : (v == 2 || v == 3 ? 184.0 : 120.0);
     p.turn[v] = p.nitems[v] > slots && rows * p.outw * cell * slots / p.nitems[v] <= L2_BYTES;
     return 0;
+}
+
+// Table v, cut for the resident CTAs of the ring its launches take: the short
+// one for the plain FP64 substep of a basin alone whose items make
+// SHORT_WAVES waves at most (us per substep with 5 and 4 slots: 4 waves,
+// 1700^2 73.7, 73.7 and 1800 x 1300 general 85.9, 85.0; 5 waves, 2048 x 1536
+// general 112, 114; 6 waves, 2048^2 102.9, 105.3).
+int build_table(Plan &p, const Dom &d, int v, int rows_per_item, cudaStream_t s)
+{
+    if (v <= 1 && p.min_rows <= 2) {
+        const int slots = p.nsm * p.occ_short[v];
+        const std::vector<int4> items = partition(p, d, slots, rows_per_item);
+        if ((long long)items.size() <= (long long)SHORT_WAVES * slots) return upload_items(p, v, items, slots, SHORT_RING, s);
+    }
+    const int slots = p.nsm * p.occ[v];
+    return upload_items(p, v, partition(p, d, slots, rows_per_item), slots, RING, s);
 }
 
 void release(Plan &p)
@@ -1638,24 +1676,22 @@ int setup(Plan &p, const Dom &d, const Consts &c, const float *const masks[7], c
     p.nsm = nsm;
     // one item table per variant for the plain substep and one for the
     // time-mean substeps, cut for the kernel's resident CTAs
-    int occ[NTABLE] = {1, 1, 1, 1, 1};
-    cudaError_t oe = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[0], k_substep<false, 3>, NL,
-                                                                   ring_bytes<false, 3>());
-    if (oe == cudaSuccess)
-        oe = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], k_substep<true, 3>, NL, ring_bytes<true, 3>());
-    if (oe == cudaSuccess)
-        oe = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], k_substep<false, 5>, NL, ring_bytes<false, 5>());
-    if (oe == cudaSuccess)
-        oe = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[3], k_substep<true, 5>, NL, ring_bytes<true, 5>());
-    if (oe == cudaSuccess)
-        oe = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[4], k_substep<false, 3, true>, NL,
-                                                           ring_bytes<false, 3, true>());
-    if (oe != cudaSuccess) return 1;
+    auto occupancy = [](int &n, const void *kernel, size_t smem) {
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, NL, smem);
+        n = std::max(n, 1);
+        return e != cudaSuccess;
+    };
+    if (occupancy(p.occ[0], (const void *)k_substep<false, 3>, ring_bytes<false, 3>()) ||
+        occupancy(p.occ[1], (const void *)k_substep<true, 3>, ring_bytes<true, 3>()) ||
+        occupancy(p.occ[2], (const void *)k_substep<false, 5>, ring_bytes<false, 5>()) ||
+        occupancy(p.occ[3], (const void *)k_substep<true, 5>, ring_bytes<true, 5>()) ||
+        occupancy(p.occ[4], (const void *)k_substep<false, 3, true>, ring_bytes<false, 3, true>()) ||
+        occupancy(p.occ_short[0], (const void *)k_substep<false, 3, false, SHORT_RING>, ring_bytes<false, 3>(SHORT_RING)) ||
+        occupancy(p.occ_short[1], (const void *)k_substep<true, 3, false, SHORT_RING>, ring_bytes<true, 3>(SHORT_RING)))
+        return 1;
     p.ocean = ocean_rows(p, d, masks[0]);
-    for (int v = 0; v < NTABLE; v++) {
-        p.occ[v] = occ[v] < 1 ? 1 : occ[v];
-        if (upload_items(p, v, partition(p, d, nsm * p.occ[v], 0), s)) return 1;
-    }
+    for (int v = 0; v < NTABLE; v++)
+        if (build_table(p, d, v, 0, s)) return 1;
     p.rows_per_item[0] = p.rows_per_item[1] = 0;
     return 0;
 }
@@ -1837,7 +1873,7 @@ int repartition(Plan &p, const Dom &d, int rows_per_item, cudaStream_t s)
 {
     for (int v = 0; v < NTABLE; v++) {
         p.rows_per_item[v & 1] = rows_per_item;
-        if (upload_items(p, v, partition(p, d, p.nsm * p.occ[v], rows_per_item), s)) return 1;
+        if (build_table(p, d, v, rows_per_item, s)) return 1;
     }
     return 0;
 }
@@ -1929,8 +1965,8 @@ int launch_step_ext(Plan &p, const Dom &d, const Consts &c, double dt, int ext_s
     if (set_io(p, q, state, p.buf[0])) return 1;
     q.items = t->items;
     p.last_variant = gen;
-    if (gen) launch_substep<true, 3>(t->nitems, q, s);
-    else launch_substep<false, 3>(t->nitems, q, s);
+    if (gen) launch_plain<true>(p.ring[1], t->nitems, q, s);
+    else launch_plain<false>(p.ring[0], t->nitems, q, s);
     if (cudaGetLastError() != cudaSuccess) return 1;
     for (int k = 0; k < 6; k++) std::swap(state[k], p.buf[0][k]);
     return 0;

@@ -91,6 +91,7 @@ struct Plan {
     // different numbers of CTAs per SM)
     int nitems[5] = {0, 0, 0, 0, 0};
     int4 *items[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // {g0, first row, end row, strip} per item
+    int ring[5] = {5, 5, 5, 5, 5};  // ring slots its launches take
     bool turn[5] = {};        // alternate substeps take a table's items from its end
     bool uni = false;         // metrics all equal one spacing d (square uniform grid)
     double d = 0.0;           // that spacing
@@ -105,6 +106,7 @@ struct Plan {
     CUtensorMap tm_set[3];          // box {36, 1, 6} over each state set
     CUtensorMap tm_stat[2];         // box {36, 1, 3 | 6} over the static block
     int occ[5] = {0, 0, 0, 0, 0};   // resident CTAs per SM, per item table
+    int occ_short[2] = {0, 0};      // the same with the short ring (plain FP64 substep)
     std::vector<uint8_t> ocean;     // per strip and interior row: any written column is ocean
     int rows_per_item[2] = {0, 0};  // 0: cut by cost (partition); else about that many rows per item
     int min_rows = 2;               // no work item is cut shorter (an ensemble member: 16)

@@ -56,3 +56,36 @@ def test_land_runs_in_the_strips(gpu, ora, nx, ny, bands, call):
     if call:
         for k, v in bo.means.items():
             assert rel_err(bg.means[k], v) <= 1e-12, k
+
+
+# a basin alone of few waves of items takes the ring of four slots, an
+# ensemble's member the ring of five: the same values bit for bit (items of
+# 1-2 rows, about 7, several waves; past four waves both take five)
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,nx,ny", [
+    ("beta", 31, 31), ("beta", 330, 330), ("beta", 1300, 1300), ("beta", 1750, 1750),
+    ("regional", 300, 200), ("spherical", 45, 33), ("spherical", 701, 487), ("spherical", 1800, 1300),
+])
+def test_ring_sizes_agree(gpu, ora, kind, nx, ny):
+    if kind == "beta":
+        b = basins.beta_plane_basin(n=nx, seed=nx)
+    elif kind == "regional":
+        b = basins.regional_basin(nx=nx, ny=ny, seed=nx)
+    else:
+        b = basins.spherical_basin(nx=nx, ny=ny, dxst=12.0 / nx, dyst=8.0 / ny, dt=2.0)
+    basins.finalize(b, ora.OracleBackend())
+    ora.hh_init_external(b)
+    b1, b2 = b.copy(), b.copy()
+    with gpu.BarotropicSolver(b1, resident=True) as s:
+        assert s.path()[0] == 1
+        s.load_state()
+        s.run_substeps(6, b.dt)
+        s.sync_to_host()
+    with gpu.BarotropicSolver(b2, resident=True) as s:
+        s.load_state()
+        with gpu.Ensemble([s], group=2) as e:
+            e.run(6, [b.dt], np.ones(6))
+        s.sync_to_host()
+    for k in STATE:
+        assert np.array_equal(b1.state[k], b2.state[k]), k
+    assert np.abs(b1.state["ubrtr_e"]).max() > 0.0
