@@ -43,7 +43,7 @@ oracle's time on the host cores (a study line).
 --study tracer times inmsom_tracer_tran_diff (one tracer's transport,
 isoneutral/GM diffusion and implicit vertical diffusion) the same way on the
 same basin and levels (a study line).
---study general times the per-loop path (the fallback of grids the fused
+--study general times the general path (the fallback of grids the fused
 kernel does not take) on the benchmark basin beside the fused path, and on
 the periodic Williamson test-2 sphere (a study line).
 --study fp32 runs the FP32-velocity variant against the FP64 run on the
@@ -516,7 +516,7 @@ def run_ours(args):
 
 
 def run_study_general(args):
-    """The per-loop path (the reference's sweeps, bit-exact rounding) that
+    """The general path (the reference's sweeps, bit-exact rounding) that
     grids the fused kernel does not take -- biharmonic viscosity, periodic
     wraps, ocean halos, metrics varying along rows -- fall back to: device
     time per step on the benchmark basin forced onto it, beside the fused
@@ -837,7 +837,7 @@ def run_study_baroclinic(args):
                      "traffic_source": "ncu dram bytes of a 512x512x20 launch scaled by cell-levels",
                      "algorithmic_bytes_per_call": int(alg),
                      "kernels_timed": "k_columns (8 row bands) + k_border, CUDA events around each launch"},
-        "gpu_launches": 9 * len(comp),            # per call: k_columns for each of 8 row bands, k_border
+        "gpu_launches": 17 * len(comp),           # per call: k_columns and k_border (the sides) for each of 8 row bands, k_border
         "clocks": clk.summary(),
     }
     if not args.no_cpu:
@@ -911,9 +911,9 @@ def run_study_tracer(args):
                      "algorithmic_bytes_per_call": int(alg),
                      "kernels_timed": "k_tracer_flux, wraps, k_tracer_solve (8 row bands) + k_tracer_border, "
                                       "CUDA events around each band"},
-        # per call: k_tracer_flux and k_tracer_solve for each of 8 row bands (and the flux
-        # wraps on a periodic basin), k_tracer_border
-        "gpu_launches": 17 * len(comp),
+        # per call: k_tracer_flux, k_tracer_solve and k_tracer_border (the sides) for each of 8
+        # row bands (and the flux wraps on a periodic basin), k_tracer_border
+        "gpu_launches": 25 * len(comp),
         "clocks": clk.summary(),
     }
     if not args.no_cpu:

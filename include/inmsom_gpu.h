@@ -611,11 +611,11 @@ int inmsom_ens_run(inmsom_ens *ens, int nsub, const double *dt, const double *rh
 /* Autotuner: for each size class of members (side length rounded to 256),
  * times `trial_groups` groups of substeps in the ensemble's current form
  * (graph or persistent: tune each form for itself) with each candidate
- * chunk height (one wave of cost-balanced chunks, or about 96, 64, 48 or 32
+ * chunk height (the default cut into cost-balanced chunks, or about 96, 64, 48 or 32
  * rows per chunk) and keeps the fastest; the combination is then timed
  * against the members' cut before tuning, which stays if it is faster.
- * rows_per_item[i] receives member i's choice (0 = one wave), which the
- * members keep.  The trial runs advance the members' states. */
+ * rows_per_item[i] receives member i's choice (0 = the default cut), which
+ * the members keep.  The trial runs advance the members' states. */
 int inmsom_ens_tune(inmsom_ens *ens, const double *dt, int trial_groups, int *rows_per_item);
 /* on != 0: inmsom_ens_run advances each group of substeps of all members
  * with ONE persistent cooperative launch (still replayed as a CUDA graph)

@@ -373,8 +373,8 @@ class Ensemble:
     def tune(self, dt, trial_groups: int = 2):
         """Autotune chunk heights per size class in the ensemble's current
         form (graph or persistent); the cut before tuning stays unless the
-        tuned one is faster.  Returns rows per item per member (0 = one wave
-        of cost-balanced chunks).  Advances the states."""
+        tuned one is faster.  Returns rows per item per member (0 = the
+        default cut into cost-balanced chunks).  Advances the states."""
         d = self._dt(dt)
         out = (ctypes.c_int * len(self.members))()
         check(load().inmsom_ens_tune(self._ens, dptr(d), int(trial_groups), out))
