@@ -232,16 +232,19 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(&s.mbar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // Launched with programmatic stream serialisation: what follows reads what
+    // earlier kernels of the stream wrote (the weights, the batch).  The
+    // tensor memory is taken only now: the stream's last kernel may be
+    // another program's that takes tensor memory after it let this one in,
+    // and would wait for columns held by a CTA that waits for its end.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    fetch(blockIdx.x);
     if (w == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&s.tmem_base)),
                      "r"(TM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // what follows reads what earlier kernels of the stream wrote (the
-    // weights, the batch): launched with programmatic stream serialisation
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    fetch(blockIdx.x);
     // weights, 16 bytes (8 outputs of one input) at a time
     {
         constexpr int G = HID / 8, N1 = KIN * G, N2 = HID * G;   // pieces
