@@ -426,6 +426,11 @@ int inmsom_gpu_path(inmsom_ctx *ctx, int *path, const char **reason);
  * Nothing faults and the context stays usable: with item = -1 the next
  * calls compute normally. */
 int inmsom_test_hold_copy(inmsom_ctx *ctx, int item, int ring_row, unsigned wait_polls);
+
+/* Test hook: the context's device buffers for packed host copies take at
+ * most `bytes` each from now on (as if the device had no more memory for
+ * them); negative: the built-in 64 MB. */
+int inmsom_test_stage_limit(inmsom_ctx *ctx, long long bytes);
 /* Device time of the phases of the last completed
  * inmsom_barotropic_dynamics, inmsom_baroclinic_dynamics,
  * inmsom_vertical_velocity or inmsom_tracer_tran_diff call (CUDA events on the context's stream):

@@ -414,6 +414,16 @@ int inmsom_test_hold_copy(inmsom_ctx *c, int item, int ring_row, unsigned wait_p
     return INMSOM_OK;
 }
 
+int inmsom_test_stage_limit(inmsom_ctx *c, long long bytes)
+{
+    if (!c) return set_err(INMSOM_EARG, "NULL context");
+    for (transfer::Stage *st : {&c->stage, &c->stage_up, &c->stage_dn}) {
+        transfer::release(*st);
+        st->limit = bytes < 0 ? transfer::STAGE_BYTES : (size_t)bytes;
+    }
+    return INMSOM_OK;
+}
+
 int inmsom_barotropic_dynamics(inmsom_ctx *c, double tau, int nstep, int ksw4, double *ubrtr_e,
                                double *ubrtrp_e, double *vbrtr_e, double *vbrtrp_e, double *ssh_e,
                                double *sshp_e, double *ubrtr_i, double *vbrtr_i,

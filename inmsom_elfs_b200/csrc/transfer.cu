@@ -19,21 +19,21 @@ namespace transfer {
 namespace {
 
 constexpr size_t PACK_BELOW = 8192;          // bytes per row
-constexpr size_t GROUP_BYTES = 64u << 20;    // a stage is reused after about this much
-constexpr int MAX_FIELDS = 16;               // fields per kernel launch
+constexpr int MAX_PIECES = 16;               // pieces per kernel launch
 constexpr int WARPS = 8;
 
+// pieces of fields: nrows rows from r0 on of nlev levels each
 struct Batch {
-    void *dev[MAX_FIELDS];
-    size_t off[MAX_FIELDS];    // in the stage
-    int nlev[MAX_FIELDS], elem[MAX_FIELDS];
+    void *dev[MAX_PIECES];     // row 0 of the piece's first level
+    size_t off[MAX_PIECES];    // in the stage
+    int nlev[MAX_PIECES], elem[MAX_PIECES], r0[MAX_PIECES], nrows[MAX_PIECES];
 };
 
-// one warp per row: field blockIdx.y, row w of nlev * nrows
+// one warp per row: piece blockIdx.y, row w of nlev * nrows
 template <bool UP>
-__global__ void __launch_bounds__(32 * WARPS) k_rows(Dom d, const __grid_constant__ Batch b, unsigned char *stage, int r0, int nrows)
+__global__ void __launch_bounds__(32 * WARPS) k_rows(Dom d, const __grid_constant__ Batch b, unsigned char *stage)
 {
-    const int f = blockIdx.y, lane = threadIdx.x & 31;
+    const int f = blockIdx.y, lane = threadIdx.x & 31, r0 = b.r0[f], nrows = b.nrows[f];
     const int nxa = d.bnd_x2 - d.bnd_x1 + 1, nya = d.bnd_y2 - d.bnd_y1 + 1;
     const long long total = (long long)b.nlev[f] * nrows;
     for (long long w = (long long)blockIdx.x * WARPS + (threadIdx.x >> 5); w < total; w += (long long)gridDim.x * WARPS) {
@@ -62,7 +62,20 @@ cudaError_t reserve(Stage &st, size_t bytes)
     return e;
 }
 
-// one field's rows between the host and its place in the stage
+size_t padded(size_t bytes) { return (bytes + 255) / 256 * 256; }
+
+// what nrows rows of the packed ones of n fields take in a stage
+size_t packed_bytes(const Dom &d, const Field *f, int n, int nrows)
+{
+    size_t bytes = 0;
+    for (int k = 0; k < n; k++) {
+        const size_t line = (size_t)d.nxa() * f[k].elem;
+        if (line < PACK_BELOW) bytes += padded(line * nrows * f[k].nlev);
+    }
+    return bytes;
+}
+
+// a piece's rows between the host and its place in the stage
 cudaError_t packed_copy(unsigned char *stage, const Dom &d, const Field &f, int r0, int nrows, bool up, cudaStream_t s)
 {
     const size_t row = (size_t)d.nxa() * f.elem, slab = row * nrows, level = row * d.nya();
@@ -112,33 +125,64 @@ cudaError_t rows(Stage &st, const Dom &d, const Field *f, int n, int r0, int r1,
 {
     const int nrows = r1 - r0 + 1;
     if (nrows < 1) return cudaSuccess;
-    cudaError_t e = cudaSuccess;
-    for (int k = 0; k < n && e == cudaSuccess;) {
-        if ((size_t)d.nxa() * f[k].elem >= PACK_BELOW) {
+    cudaError_t e = reserve(st, std::min(packed_bytes(d, f, n, nrows), st.limit));
+    int k = 0, lev = 0, row = r0;   // the next field, and the level and row it goes on with
+    while (k < n && e == cudaSuccess) {
+        const size_t line = (size_t)d.nxa() * f[k].elem;
+        if (line < PACK_BELOW && line > st.cap) return cudaErrorMemoryAllocation;
+        if (line >= PACK_BELOW) {
             e = pitched_copy(d, f[k++], r0, nrows, up, s);
             continue;
         }
+        // fill the stage: whole fields, and of one too large for it runs of
+        // levels (or of a level's rows)
         Batch b = {};
-        size_t bytes = 0;
-        int m = 0, tall = 1;
-        for (; k + m < n && m < MAX_FIELDS && (m == 0 || bytes < GROUP_BYTES); m++) {
-            const Field &g = f[k + m];
-            if ((size_t)d.nxa() * g.elem >= PACK_BELOW) break;
-            b.dev[m] = g.dev;
-            b.off[m] = bytes;
-            b.nlev[m] = g.nlev;
+        Field part[MAX_PIECES];
+        size_t used = 0;
+        int m = 0;
+        long long tall = 1;
+        for (; k < n && m < MAX_PIECES; m++) {
+            const Field &g = f[k];
+            const size_t line = (size_t)d.nxa() * g.elem, slab = line * nrows, room = st.cap - used;
+            if (line >= PACK_BELOW || line > st.cap) break;
+            int levels = g.nlev - lev, lines = nrows;
+            if (row != r0 || slab * levels > room) {
+                if (m > 0) break;
+                if (row == r0 && slab <= room) {
+                    levels = (int)(room / slab);
+                } else {
+                    levels = 1;
+                    lines = (int)std::min<size_t>(r1 - row + 1, room / line);
+                }
+            }
+            const size_t above = (size_t)lev * d.nya();   // rows of the levels before
+            part[m] = Field{(unsigned char *)g.dev + above * d.pitch * g.elem, (unsigned char *)g.host + above * line, levels,
+                            g.elem};
+            b.dev[m] = part[m].dev;
+            b.off[m] = used;
+            b.nlev[m] = levels;
             b.elem[m] = g.elem;
-            tall = std::max(tall, g.nlev);
-            bytes += ((size_t)d.nxa() * g.elem * nrows * g.nlev + 255) / 256 * 256;
+            b.r0[m] = row;
+            b.nrows[m] = lines;
+            tall = std::max(tall, (long long)levels * lines);
+            used = std::min(st.cap, used + padded(line * lines * levels));
+            if (lines == nrows) {
+                lev += levels;
+            } else if ((row += lines) > r1) {
+                row = r0;
+                lev++;
+            }
+            if (lev == g.nlev) {
+                lev = 0;
+                k++;
+            }
         }
-        if ((e = reserve(st, bytes)) != cudaSuccess) break;
         unsigned char *stage = (unsigned char *)st.p;
-        const dim3 grid((unsigned)std::min<long long>(((long long)nrows * tall + WARPS - 1) / WARPS, 1 << 16), m);
-        if (!up) k_rows<false><<<grid, 32 * WARPS, 0, s>>>(d, b, stage, r0, nrows);
-        for (int q = 0; q < m && e == cudaSuccess; q++) e = packed_copy(stage + b.off[q], d, f[k + q], r0, nrows, up, s);
-        if (up && e == cudaSuccess) k_rows<true><<<grid, 32 * WARPS, 0, s>>>(d, b, stage, r0, nrows);
+        const dim3 grid((unsigned)std::min<long long>((tall + WARPS - 1) / WARPS, 1 << 16), m);
+        if (!up) k_rows<false><<<grid, 32 * WARPS, 0, s>>>(d, b, stage);
+        for (int q = 0; q < m && e == cudaSuccess; q++) e = packed_copy(stage + b.off[q], d, part[q], b.r0[q], b.nrows[q], up, s);
+        if (up && e == cudaSuccess) k_rows<true><<<grid, 32 * WARPS, 0, s>>>(d, b, stage);
         if (e == cudaSuccess) e = cudaGetLastError();
-        k += m;
     }
     return e;
 }
@@ -146,7 +190,8 @@ cudaError_t rows(Stage &st, const Dom &d, const Field *f, int n, int r0, int r1,
 void release(Stage &st)
 {
     cudaFree(st.p);
-    st = Stage{};
+    st.p = nullptr;
+    st.cap = 0;
 }
 
 }  // namespace transfer

@@ -19,10 +19,14 @@ struct Field {
 };
 
 // packed device copy of rows on their way; owned by a context, used on one
-// stream, grown on demand
+// stream, grown on demand to STAGE_BYTES at most: more than that goes through
+// it in several turns (a turn costs a kernel launch, some microseconds
+// against the millisecond that 64 MB take on the host link)
+constexpr size_t STAGE_BYTES = 64u << 20;
 struct Stage {
     void *p = nullptr;
     size_t cap = 0;
+    size_t limit = STAGE_BYTES;
 };
 
 // rows r0..r1 (0-based from bnd_y1), whole rows of every level of n fields,
