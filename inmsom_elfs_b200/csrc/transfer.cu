@@ -8,7 +8,8 @@
 // long pieces brings it to a packed stage on the device, and one kernel for
 // all fields moves it into the pitched rows (or out of them), at HBM speed.
 // Longer rows are copied pitched, which needs neither the stage nor the
-// extra pass over memory (16 KB rows: 51 GB/s of the link's 55).
+// extra pass over memory (16 KB rows: 51 GB/s of the link's 55); so are all
+// rows when the device has no memory left for a stage.
 #include "transfer.h"
 
 #include <algorithm>
@@ -52,14 +53,23 @@ __global__ void __launch_bounds__(32 * WARPS) k_rows(Dom d, const __grid_constan
     }
 }
 
+// room for `bytes`, as far as the limit and the device's memory go: a stage
+// that cannot grow stays as it is
 cudaError_t reserve(Stage &st, size_t bytes)
 {
+    bytes = std::min(bytes, st.limit);
     if (bytes <= st.cap) return cudaSuccess;
+    void *p = nullptr;
+    const cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        return cudaSuccess;
+    }
+    if (e != cudaSuccess) return e;
     release(st);
-    const cudaError_t e = cudaMalloc(&st.p, bytes);
-    if (e == cudaSuccess) st.cap = bytes;
-    else st.p = nullptr;
-    return e;
+    st.p = p;
+    st.cap = bytes;
+    return cudaSuccess;
 }
 
 size_t padded(size_t bytes) { return (bytes + 255) / 256 * 256; }
@@ -125,12 +135,11 @@ cudaError_t rows(Stage &st, const Dom &d, const Field *f, int n, int r0, int r1,
 {
     const int nrows = r1 - r0 + 1;
     if (nrows < 1) return cudaSuccess;
-    cudaError_t e = reserve(st, std::min(packed_bytes(d, f, n, nrows), st.limit));
+    cudaError_t e = reserve(st, packed_bytes(d, f, n, nrows));
     int k = 0, lev = 0, row = r0;   // the next field, and the level and row it goes on with
     while (k < n && e == cudaSuccess) {
         const size_t line = (size_t)d.nxa() * f[k].elem;
-        if (line < PACK_BELOW && line > st.cap) return cudaErrorMemoryAllocation;
-        if (line >= PACK_BELOW) {
+        if (line >= PACK_BELOW || line > st.cap) {
             e = pitched_copy(d, f[k++], r0, nrows, up, s);
             continue;
         }

@@ -1,8 +1,10 @@
 """The device buffer that packed host copies go through: its size is bounded,
 whatever the fields' size, and fields larger than it go through it in runs of
-levels, or of a level's rows."""
+levels, or of a level's rows.  A device without the memory for it (here: a
+limit below one row) takes the pitched copies."""
 import numpy as np
 import pytest
+from conftest import rel_err
 
 from inmsom_elfs_b200 import _lib, basins
 from test_baroclinic import TAU, _run_oracle, coastline, inputs
@@ -73,6 +75,23 @@ def test_small_stages_banded(gpu, ora, limit):
         got = _baroclinic(sol, dz, hzt, f)
     for g, w in zip(got, want):
         assert np.array_equal(g, w)
+
+
+@pytest.mark.parametrize("limit", [0, 1, 271])
+def test_no_memory_for_a_stage(gpu, ora, limit):
+    b = coastline(ora, nx=30, ny=20, seed=5)
+    ora.hh_init_external(b)
+    with gpu.BarotropicSolver(b) as sol:
+        assert _lib.load().inmsom_test_stage_limit(sol._ctx, limit) == _lib.OK
+        _depth_ave(b, sol, 5, limit)
+        dz, hzt, f = inputs(b, nz=4, seed=9)
+        for g, w in zip(_baroclinic(sol, dz, hzt, f), _run_oracle(ora, b, dz, hzt, f)):
+            assert np.array_equal(g, w)
+        bo = b.copy()
+        sol.barotropic_dynamics(2 * b.dt, 2)
+        ora.barotropic_dynamics(bo, 2 * b.dt, 2)
+        for k, v in bo.state.items():
+            assert rel_err(b.state[k], v) <= 1e-12, k
 
 
 def test_stage_limit_argument_checks():
