@@ -431,6 +431,8 @@ int inmsom_test_hold_copy(inmsom_ctx *ctx, int item, int ring_row, unsigned wait
  * most `bytes` each from now on (as if the device had no more memory for
  * them); negative: the built-in 64 MB. */
 int inmsom_test_stage_limit(inmsom_ctx *ctx, long long bytes);
+/* ... and how often they were allocated so far */
+int inmsom_test_stage_allocs(inmsom_ctx *ctx, int *count);
 /* Device time of the phases of the last completed
  * inmsom_barotropic_dynamics, inmsom_baroclinic_dynamics,
  * inmsom_vertical_velocity or inmsom_tracer_tran_diff call (CUDA events on the context's stream):

@@ -424,6 +424,13 @@ int inmsom_test_stage_limit(inmsom_ctx *c, long long bytes)
     return INMSOM_OK;
 }
 
+int inmsom_test_stage_allocs(inmsom_ctx *c, int *count)
+{
+    if (!c || !count) return set_err(INMSOM_EARG, "NULL argument");
+    *count = c->stage.allocs + c->stage_up.allocs + c->stage_dn.allocs;
+    return INMSOM_OK;
+}
+
 int inmsom_barotropic_dynamics(inmsom_ctx *c, double tau, int nstep, int ksw4, double *ubrtr_e,
                                double *ubrtrp_e, double *vbrtr_e, double *vbrtrp_e, double *ssh_e,
                                double *sshp_e, double *ubrtr_i, double *vbrtr_i,

@@ -79,6 +79,22 @@ int pipelined(inmsom_ctx *c, int nb, const std::vector<Field> &pre, const double
     auto down = [&](int r0, int r1) {
         return transfer::rows(c->stage_dn, d, out.data(), (int)out.size(), r0, r1, false, c->s_dn);
     };
+    // band b: interior rows first(b) .. first(b+1)-1, uploaded up to (not
+    // including) array row up_end(b)
+    auto first = [&](int b) { return d.ny_start + (int)((long long)nyi * b / nb); };
+    auto up_end = [&](int b) { return b == nb - 1 ? nya : first(b + 1) + 1 - d.bnd_y1; };
+    // both stages at the largest band's size before the first copy: to grow
+    // one later would wait for the copies under way
+    int most_up = 0, most_dn = std::max(iy0, nya - 1 - iy1);
+    for (int b = 0; b < nb; b++) {
+        most_up = std::max(most_up, up_end(b) - (b ? up_end(b - 1) : 0));
+        most_dn = std::max(most_dn, first(b + 1) - first(b));
+    }
+    auto bytes = [&](const std::vector<Field> &f, int nrows) {
+        return transfer::packed_bytes(d, f.data(), (int)f.size(), nrows);
+    };
+    CK(transfer::reserve(c->stage_up, std::max(bytes(pre, nya), bytes(in, most_up))));
+    CK(transfer::reserve(c->stage_dn, bytes(out, most_dn)));
     c->ph_valid = false;
     c->ph_direct = false;
     CK(cudaEventRecord(c->ph[0], c->stream));
@@ -86,13 +102,9 @@ int pipelined(inmsom_ctx *c, int nb, const std::vector<Field> &pre, const double
     CK(cudaMemcpyAsync(lev, dz, nz * sizeof(double), cudaMemcpyHostToDevice, c->s_up));
     CK(cudaMemcpyAsync(lev + nz, hzt, (nz + 1) * sizeof(double), cudaMemcpyHostToDevice, c->s_up));
     CK(up(pre, 0, nya - 1));
-    int up_next = 0;
     for (int b = 0; b < nb; b++) {
-        const int n0 = d.ny_start + (int)((long long)nyi * b / nb);
-        const int n1 = d.ny_start + (int)((long long)nyi * (b + 1) / nb) - 1;
-        const int up_last = b == nb - 1 ? nya - 1 : n1 + 1 - d.bnd_y1;
-        CK(up(in, up_next, up_last));
-        up_next = up_last + 1;
+        const int n0 = first(b), n1 = first(b + 1) - 1;
+        CK(up(in, b ? up_end(b - 1) : 0, up_end(b) - 1));
         CK(cudaEventRecord(ev_up[b], c->s_up));
         CK(cudaStreamWaitEvent(c->stream, ev_up[b], 0));
         CK(cudaEventRecord(ev_k0[b], c->stream));

@@ -178,6 +178,11 @@ class Copies {
     std::vector<transfer::Field> f;
     int go(bool to_device)
     {
+        // one allocation for the life of the context: the largest 2-D call
+        // moves the state, the scratch, the forcing and the depths
+        constexpr size_t most = NSTATE + NSCR + NFORC + NDEPTH;
+        const transfer::Field one{nullptr, nullptr, 1, (int)sizeof(double)};
+        CK(transfer::reserve(c->stage, most * transfer::packed_bytes(c->dom, &one, 1, c->dom.nya())));
         CK(transfer::rows(c->stage, c->dom, f.data(), (int)f.size(), 0, c->dom.nya() - 1, to_device, c->stream));
         f.clear();
         return INMSOM_OK;

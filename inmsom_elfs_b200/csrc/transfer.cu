@@ -53,37 +53,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rows(Dom d, const __grid_constan
     }
 }
 
-// room for `bytes`, as far as the limit and the device's memory go: a stage
-// that cannot grow stays as it is
-cudaError_t reserve(Stage &st, size_t bytes)
-{
-    bytes = std::min(bytes, st.limit);
-    if (bytes <= st.cap) return cudaSuccess;
-    void *p = nullptr;
-    const cudaError_t e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation) {
-        (void)cudaGetLastError();
-        return cudaSuccess;
-    }
-    if (e != cudaSuccess) return e;
-    release(st);
-    st.p = p;
-    st.cap = bytes;
-    return cudaSuccess;
-}
-
 size_t padded(size_t bytes) { return (bytes + 255) / 256 * 256; }
-
-// what nrows rows of the packed ones of n fields take in a stage
-size_t packed_bytes(const Dom &d, const Field *f, int n, int nrows)
-{
-    size_t bytes = 0;
-    for (int k = 0; k < n; k++) {
-        const size_t line = (size_t)d.nxa() * f[k].elem;
-        if (line < PACK_BELOW) bytes += padded(line * nrows * f[k].nlev);
-    }
-    return bytes;
-}
 
 // a piece's rows between the host and its place in the stage
 cudaError_t packed_copy(unsigned char *stage, const Dom &d, const Field &f, int r0, int nrows, bool up, cudaStream_t s)
@@ -130,6 +100,34 @@ cudaError_t pitched_copy(const Dom &d, const Field &f, int r0, int nrows, bool u
 }
 
 }  // namespace
+
+size_t packed_bytes(const Dom &d, const Field *f, int n, int nrows)
+{
+    size_t bytes = 0;
+    for (int k = 0; k < n; k++) {
+        const size_t line = (size_t)d.nxa() * f[k].elem;
+        if (line < PACK_BELOW) bytes += padded(line * nrows * f[k].nlev);
+    }
+    return bytes;
+}
+
+cudaError_t reserve(Stage &st, size_t bytes)
+{
+    bytes = std::min(bytes, st.limit);
+    if (bytes <= st.cap) return cudaSuccess;
+    void *p = nullptr;
+    const cudaError_t e = cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        return cudaSuccess;
+    }
+    if (e != cudaSuccess) return e;
+    release(st);
+    st.p = p;
+    st.cap = bytes;
+    st.allocs++;
+    return cudaSuccess;
+}
 
 cudaError_t rows(Stage &st, const Dom &d, const Field *f, int n, int r0, int r1, bool up, cudaStream_t s)
 {

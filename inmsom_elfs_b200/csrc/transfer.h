@@ -19,7 +19,7 @@ struct Field {
 };
 
 // packed device copy of rows on their way; owned by a context, used on one
-// stream, grown on demand to STAGE_BYTES at most: more than that goes through
+// stream, grown to STAGE_BYTES at most: more than that goes through
 // it in several turns (a turn costs a kernel launch, some microseconds
 // against the millisecond that 64 MB take on the host link)
 constexpr size_t STAGE_BYTES = 64u << 20;
@@ -27,7 +27,15 @@ struct Stage {
     void *p = nullptr;
     size_t cap = 0;
     size_t limit = STAGE_BYTES;
+    int allocs = 0;            // allocations so far
 };
+
+// what rows needs a stage to hold for nrows rows of n fields at once
+size_t packed_bytes(const Dom &d, const Field *f, int n, int nrows);
+// room for `bytes`, as far as the limit and the device's memory go: a stage
+// that cannot grow stays as it is.  Growing waits for the device, so that a
+// caller who knows what is to come reserves it first
+cudaError_t reserve(Stage &st, size_t bytes);
 
 // rows r0..r1 (0-based from bnd_y1), whole rows of every level of n fields,
 // to the device (up) or to the host, enqueued on s

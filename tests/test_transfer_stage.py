@@ -2,6 +2,8 @@
 whatever the fields' size, and fields larger than it go through it in runs of
 levels, or of a level's rows.  A device without the memory for it (here: a
 limit below one row) takes the pitched copies."""
+import ctypes
+
 import numpy as np
 import pytest
 from conftest import rel_err
@@ -94,5 +96,30 @@ def test_no_memory_for_a_stage(gpu, ora, limit):
             assert rel_err(b.state[k], v) <= 1e-12, k
 
 
+@pytest.mark.parametrize("nx,ny", [(5, 4), (30, 20), (90, 43), (400, 300)])
+def test_stages_are_allocated_once(gpu, ora, nx, ny):
+    """One allocation serves every 2-D copy of a context, one per direction
+    the bands of a 3-D call (the last band is the tallest)."""
+    b = coastline(ora, nx=nx, ny=ny, seed=5)
+    ora.hh_init_external(b)
+
+    def allocs():
+        n = ctypes.c_int()
+        assert _lib.load().inmsom_test_stage_allocs(sol._ctx, ctypes.byref(n)) == _lib.OK
+        return n.value
+
+    with gpu.BarotropicSolver(b) as sol:
+        assert allocs() == 1
+        sol.load_state()
+        sol.barotropic_dynamics(2 * b.dt, 2, 1)
+        assert allocs() == 1
+        dz, hzt, f = inputs(b, nz=4, seed=9)
+        _baroclinic(sol, dz, hzt, f)
+        assert allocs() == 3
+        _baroclinic(sol, dz, hzt, f)
+        assert allocs() == 3
+
+
 def test_stage_limit_argument_checks():
     assert _lib.load().inmsom_test_stage_limit(None, 0) == _lib.EARG
+    assert _lib.load().inmsom_test_stage_allocs(None, None) == _lib.EARG
