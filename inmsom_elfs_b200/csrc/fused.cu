@@ -417,7 +417,8 @@ using On = std::integral_constant<bool, B>;
 // write 1 stores the new state
 template <bool GEN, int MODE, bool F32 = false, int RS = RING>
 __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap *tm_src, double *const *dst,
-                                             const double rs, const int4 item, unsigned char *ring, uint64_t *mbar)
+                                             const double rs, const int4 item, const int index, unsigned char *ring,
+                                             uint64_t *mbar)
 {
     using L = Layout<GEN, F32>;
     constexpr int ACC = MODE % 3;
@@ -438,7 +439,7 @@ __device__ __forceinline__ bool substep_item(const Params &p, const CUtensorMap 
 #define AT(o, f, dk) (*reinterpret_cast<const double *>(lane + (o) + L::STAT_OFF + ((f) * SEG + (dk)) * 8))
 #define CF(o, x) (reinterpret_cast<const RowCoef *>(ring + (o) + L::COEF_OFF)->x)
 
-    const int hold = (int)blockIdx.x == p.hold_item ? min(row_lo + p.hold_row, row_hi) : -1;   // test hook
+    const int hold = index == p.hold_item ? min(row_lo + p.hold_row, row_hi) : -1;   // test hook
     auto issue = [&](int row, int slot) {
         if (row == hold) return;
         issue_row<GEN, F32>(ring + slot * L::SLOT_B, &mbar[slot], tm_src, &p.tm_stat, &p.tm_ssh, &p.tm_rhs, p.rows + row,
@@ -829,7 +830,8 @@ __global__ void __launch_bounds__(NL, min_ctas<GEN, MODE, F32>()) k_substep(cons
     }
     uint64_t *mbar = reinterpret_cast<uint64_t *>(ring + RS * L::SLOT_B);
     const double rs = p.rs_dev ? p.rs_dev[*p.rs_base + p.rs_k] : p.rhs_scale;
-    (void)substep_item<GEN, MODE, F32, RS>(p, &p.tm_src, p.dst, rs, p.items[p.turn ? gridDim.x - 1 - blockIdx.x : blockIdx.x], ring, mbar);
+    const int index = p.turn ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+    (void)substep_item<GEN, MODE, F32, RS>(p, &p.tm_src, p.dst, rs, p.items[index], index, ring, mbar);
 }
 
 // ---------------------------------------------------------------------
@@ -915,10 +917,10 @@ __global__ void __launch_bounds__(NL, ens_ctas<ANYGEN>())
         const int4 item = em.items[mi.y];
         if (ANYGEN && em.gen) {
             uint64_t *mbar = reinterpret_cast<uint64_t *>(ring + RING * Layout<true>::SLOT_B);
-            (void)substep_item<true, 3>(q, &q.tm_src, q.dst, rs, item, ring, mbar);
+            (void)substep_item<true, 3>(q, &q.tm_src, q.dst, rs, item, mi.y, ring, mbar);
         } else {
             uint64_t *mbar = reinterpret_cast<uint64_t *>(ring + RING * Layout<false>::SLOT_B);
-            (void)substep_item<false, 3>(q, &q.tm_src, q.dst, rs, item, ring, mbar);
+            (void)substep_item<false, 3>(q, &q.tm_src, q.dst, rs, item, mi.y, ring, mbar);
         }
         // this item's stores, visible to the bulk copies of later items, then counted
         asm volatile("fence.proxy.async;" ::: "memory");
