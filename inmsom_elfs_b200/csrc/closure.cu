@@ -153,7 +153,7 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p)
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// layers 2 and 3 take 2 GELU (gelu2) as their input: their weights are
+// layers 2 and 3 take 2 GELU (gelu2_pair) as their input: their weights are
 // halved here (exact in BF16), so that every product is the network's.
 // Weights that do not start on 16 bytes are read one by one.
 __device__ __forceinline__ void load_weights(Weights &s, const __nv_bfloat16 *wb, const float *prm)
@@ -287,7 +287,7 @@ __device__ __forceinline__ void bias(float acc[8][4], const float *b)
 
 // y (outputs 0, 1 of cells g and g+8 in o[0..3] of lanes t == 0) of the
 // 16 cells whose layer-1 A fragments are a1.  The hidden activations are
-// kept as 2 GELU (gelu2), the weights of layers 2 and 3 halved: the same
+// kept as 2 GELU (gelu2_pair), the weights of layers 2 and 3 halved: the same
 // products, one multiplication fewer per activation.
 __device__ __forceinline__ void mlp16(const Weights &s, const uint32_t a1[3][4], float o[4])
 {

@@ -191,15 +191,6 @@ __device__ __forceinline__ void st_chunk(__nv_bfloat16 *tile, int r, int c0, int
     *reinterpret_cast<uint4 *>(tile + blk(r, c0, C)) = q;
 }
 
-// GELU and its derivative with one hyperbolic tangent: the values of gelu
-// and gelu_d (gelu.cuh)
-__device__ __forceinline__ void gelu_both(float x, float &y, float &d)
-{
-    const float x2 = x * x, t = tanh_hw(x * fmaf(GELU_C1, x2, GELU_C0)), h = 0.5f * x;
-    y = fmaf(h, t, h);
-    d = fmaf(0.5f, 1.0f + t, h * (1.0f - t * t) * fmaf(3.0f * GELU_C1, x2, GELU_C0));
-}
-
 __global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
     k_mlp_grad_tc(const __nv_bfloat16 *__restrict__ x, const float *__restrict__ tgt, const int *__restrict__ idx,
                   int batch, const float *__restrict__ prm, const __nv_bfloat16 *__restrict__ wb,

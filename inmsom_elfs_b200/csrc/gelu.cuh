@@ -2,10 +2,12 @@
 // (2016), x * g(x) with the gate g(x) = 0.5 (1 + tanh(sqrt(2/pi)(x +
 // 0.044715 x^3))), the gate through the hardware tanh (tanh.approx.f32,
 // relative error about 2^-11: below the BF16 rounding, 2^-9, of the
-// activations).  Training (closure_tc.cu) and inference (closure.cu) use
-// this one definition, so the network the kernels train is the one they
-// run.  gelu_d is its derivative, g + x g' with
-// g' = 0.5 (1 - t^2) (sqrt(2/pi) + 3 * 0.044715 sqrt(2/pi) x^2), t the tanh.
+// activations).  Two forms of the one definition, so that the network the
+// training kernel (closure_tc.cu) trains is the one that inference
+// (closure.cu) runs: gelu_both, the value with its derivative g + x g',
+// g' = 0.5 (1 - t^2) (sqrt(2/pi) + 3 * 0.044715 sqrt(2/pi) x^2), t the tanh,
+// for training, and gelu2_pair, twice the value of two numbers, for
+// inference.
 #pragma once
 
 namespace inmsom {
@@ -20,23 +22,11 @@ __device__ __forceinline__ float tanh_hw(float x)
     return y;
 }
 
-__device__ __forceinline__ float gelu(float x)
-{
-    const float h = 0.5f * x;
-    return fmaf(h, tanh_hw(x * fmaf(GELU_C1, x * x, GELU_C0)), h);
-}
-
-// 2 GELU(x) = x (1 + t), one multiplication fewer than GELU itself and
-// bit for bit twice its value (a power-of-two scale commutes with the
-// rounding): the inference kernel feeds it to the next layer with that
-// layer's weights halved, which leaves every product a * w unchanged
-__device__ __forceinline__ float gelu2(float x)
-{
-    return fmaf(x, tanh_hw(x * fmaf(GELU_C1, x * x, GELU_C0)), x);
-}
-
-// gelu2 of two values at once, in the two-wide FP32 instructions (each half
-// rounds as the single one does)
+// 2 GELU = x (1 + t) of two values at once, in the two-wide FP32
+// instructions: one multiplication fewer than GELU itself and bit for bit
+// twice its value (a power-of-two scale commutes with the rounding).  The
+// inference kernel feeds it to the next layer with that layer's weights
+// halved, which leaves every product a * w unchanged
 __device__ __forceinline__ void gelu2_pair(float &x, float &y)
 {
     asm("{\n\t.reg .b64 v, q, c0, c1;\n\t.reg .f32 a, b;\n\t"
@@ -48,10 +38,12 @@ __device__ __forceinline__ void gelu2_pair(float &x, float &y)
         : "f"(GELU_C0), "f"(GELU_C1));
 }
 
-__device__ __forceinline__ float gelu_d(float x)
+// GELU and its derivative with one hyperbolic tangent (the training kernel)
+__device__ __forceinline__ void gelu_both(float x, float &y, float &d)
 {
-    const float x2 = x * x, t = tanh_hw(x * fmaf(GELU_C1, x2, GELU_C0));
-    return fmaf(0.5f, 1.0f + t, 0.5f * x * (1.0f - t * t) * fmaf(3.0f * GELU_C1, x2, GELU_C0));
+    const float x2 = x * x, t = tanh_hw(x * fmaf(GELU_C1, x2, GELU_C0)), h = 0.5f * x;
+    y = fmaf(h, t, h);
+    d = fmaf(0.5f, 1.0f + t, h * (1.0f - t * t) * fmaf(3.0f * GELU_C1, x2, GELU_C0));
 }
 
 }  // namespace closure
