@@ -1256,20 +1256,20 @@ constexpr int GAP_ROWS = 8;     // longest run of land rows inside an item
 constexpr double WARM = 2.5;    // an item's warm-up iterations, in ocean rows
 constexpr int WAVE_ROWS = 10, MAX_WAVES = 8;
 
-std::vector<int4> partition(const Plan &p, const Dom &d, int slots, int rows_per_item, int rf, int rl)
+struct Segment {
+    int strip, r0, r1;          // rows r0..r1, the first and last with ocean
+    double cost;
+    int n;                      // chunks (cut_segments)
+};
+
+std::vector<Segment> segments(const Plan &p, const Dom &d, int rf, int rl)
 {
-    struct Segment {
-        int strip, r0, r1;          // rows r0..r1, the first and last with ocean
-        double cost;
-        int n;
-    };
-    const int nya = d.nya();
-    auto ocean = [&](int s, int r) { return p.ocean[(size_t)s * nya + r] != 0; };
     std::vector<Segment> seg;
     for (int s = 0; s < p.nstrips; s++) {
+        const uint8_t *ocean = p.ocean.data() + (size_t)s * d.nya();
         int land = GAP_ROWS + 1;
         for (int r = rf; r <= rl; r++) {
-            if (!ocean(s, r)) {
+            if (!ocean[r]) {
                 land++;
                 continue;
             }
@@ -1280,45 +1280,60 @@ std::vector<int4> partition(const Plan &p, const Dom &d, int slots, int rows_per
             land = 0;
         }
     }
-    std::vector<int4> items;
-    if (seg.empty()) {              // no ocean: one item that writes nothing
-        items.push_back(make_int4(0, rf, rf + 1, 0));
-        return items;
-    }
-    long long rows = 0;
+    return seg;
+}
+
+std::vector<Segment> segments(const Plan &p, const Dom &d)
+{
+    return segments(p, d, d.ny_start - d.bnd_y1, d.ny_end - d.bnd_y1);
+}
+
+// the chunks of each segment; returns how many in all
+long long cut_segments(const Plan &p, std::vector<Segment> &seg, int slots, int rows_per_item)
+{
+    long long rows = 0, all = 0;
     for (const Segment &g : seg) rows += g.r1 - g.r0 + 1;
     const int min_rows = p.min_rows <= 2 && rows <= slots * 3LL / 4 ? 1 : std::max(1, p.min_rows);
     auto most = [&](const Segment &g) { return std::max(1, (g.r1 - g.r0 + 1) / min_rows); };
     if (rows_per_item > 0) {
-        for (Segment &g : seg)
+        for (Segment &g : seg) {
             g.n = std::min(most(g), std::max(1, (g.r1 - g.r0 + 1 + rows_per_item / 2) / rows_per_item));
-    } else {
-        const long long waves = std::min<long long>(MAX_WAVES, std::max<long long>(1, std::llround((double)rows / slots / WAVE_ROWS)));
-        // chunks per segment at a cost per chunk of at most t (bisection)
-        auto cut = [&](double t) {
-            long long all = 0;
-            for (Segment &g : seg) {
-                g.n = std::min(most(g), std::max(1, (int)std::ceil(g.cost / std::max(t - WARM, 1e-3))));
-                all += g.n;
-            }
-            return all;
-        };
-        double lo = WARM, hi = WARM + 1.0;
-        for (const Segment &g : seg) hi = std::max(hi, WARM + g.cost);
-        for (int k = 0; k < 48; k++) {
-            const double t = 0.5 * (lo + hi);
-            if (cut(t) <= waves * slots) hi = t;
-            else lo = t;
+            all += g.n;
         }
-        (void)cut(hi);
+        return all;
     }
-    // cut each segment at equal shares of its cumulative cost
+    const long long waves = std::min<long long>(MAX_WAVES, std::max<long long>(1, std::llround((double)rows / slots / WAVE_ROWS)));
+    // chunks per segment at a cost per chunk of at most t (bisection)
+    auto cut = [&](double t) {
+        all = 0;
+        for (Segment &g : seg) {
+            g.n = std::min(most(g), std::max(1, (int)std::ceil(g.cost / std::max(t - WARM, 1e-3))));
+            all += g.n;
+        }
+        return all;
+    };
+    double lo = WARM, hi = WARM + 1.0;
+    for (const Segment &g : seg) hi = std::max(hi, WARM + g.cost);
+    for (int k = 0; k < 48; k++) {
+        const double t = 0.5 * (lo + hi);
+        if (cut(t) <= waves * slots) hi = t;
+        else lo = t;
+    }
+    return cut(hi);
+}
+
+// each segment's chunks, at equal shares of its cumulative cost
+std::vector<int4> work_items(const Plan &p, const Dom &d, const std::vector<Segment> &seg, int rf)
+{
+    std::vector<int4> items;
+    if (seg.empty()) items.push_back(make_int4(0, rf, rf + 1, 0));   // no ocean: one item that writes nothing
     for (const Segment &g : seg) {
+        const uint8_t *ocean = p.ocean.data() + (size_t)g.strip * d.nya();
         const double share = g.cost / g.n;
         double acc = 0.0;
         int start = g.r0, made = 0;
         for (int r = g.r0; r <= g.r1; r++) {
-            acc += ocean(g.strip, r) ? 1.0 : LAND_COST;
+            acc += ocean[r] ? 1.0 : LAND_COST;
             // the rows left always suffice for the chunks left: cut at the
             // latest when there is one row for each
             const bool cut = made < g.n - 1 && (acc >= share * (made + 1) || g.r1 - r <= g.n - 1 - made);
@@ -1330,11 +1345,6 @@ std::vector<int4> partition(const Plan &p, const Dom &d, int slots, int rows_per
         }
     }
     return items;
-}
-
-std::vector<int4> partition(const Plan &p, const Dom &d, int slots, int rows_per_item)
-{
-    return partition(p, d, slots, rows_per_item, d.ny_start - d.bnd_y1, d.ny_end - d.bnd_y1);
 }
 
 constexpr double L2_BYTES = 126e6;
@@ -1375,15 +1385,20 @@ int upload_items(Plan &p, int v, const std::vector<int4> &items, int slots, int 
 // SHORT_WAVES waves at most (us per substep with 5 and 4 slots: 4 waves,
 // 1700^2 73.7, 73.7 and 1800 x 1300 general 85.9, 85.0; 5 waves, 2048 x 1536
 // general 112, 114; 6 waves, 2048^2 102.9, 105.3).
-int build_table(Plan &p, const Dom &d, int v, int rows_per_item, cudaStream_t s)
+int build_table(Plan &p, const Dom &d, int v, std::vector<Segment> &seg, int rows_per_item, cudaStream_t s)
 {
+    int ring = RING, slots = p.nsm * p.occ[v];
     if (v <= 1 && p.min_rows <= 2) {
-        const int slots = p.nsm * p.occ_short[v];
-        const std::vector<int4> items = partition(p, d, slots, rows_per_item);
-        if ((long long)items.size() <= (long long)SHORT_WAVES * slots) return upload_items(p, v, items, slots, SHORT_RING, s);
+        ring = SHORT_RING;
+        slots = p.nsm * p.occ_short[v];
     }
-    const int slots = p.nsm * p.occ[v];
-    return upload_items(p, v, partition(p, d, slots, rows_per_item), slots, RING, s);
+    const long long n = cut_segments(p, seg, slots, rows_per_item);
+    if (ring == SHORT_RING && n > (long long)SHORT_WAVES * slots) {
+        ring = RING;
+        slots = p.nsm * p.occ[v];
+        (void)cut_segments(p, seg, slots, rows_per_item);
+    }
+    return upload_items(p, v, work_items(p, d, seg, d.ny_start - d.bnd_y1), slots, ring, s);
 }
 
 void release(Plan &p)
@@ -1692,8 +1707,9 @@ int setup(Plan &p, const Dom &d, const Consts &c, const float *const masks[7], c
         occupancy(p.occ_short[1], (const void *)k_substep<true, 3, false, SHORT_RING>, ring_bytes<true, 3>(SHORT_RING)))
         return 1;
     p.ocean = ocean_rows(p, d, masks[0]);
+    std::vector<Segment> seg = segments(p, d);
     for (int v = 0; v < NTABLE; v++)
-        if (build_table(p, d, v, 0, s)) return 1;
+        if (build_table(p, d, v, seg, 0, s)) return 1;
     p.rows_per_item[0] = p.rows_per_item[1] = 0;
     return 0;
 }
@@ -1873,9 +1889,10 @@ int finish_steps_f32(Plan &p, const Dom &d, double *state[6], cudaStream_t s)
 
 int repartition(Plan &p, const Dom &d, int rows_per_item, cudaStream_t s)
 {
+    std::vector<Segment> seg = segments(p, d);
     for (int v = 0; v < NTABLE; v++) {
         p.rows_per_item[v & 1] = rows_per_item;
-        if (build_table(p, d, v, rows_per_item, s)) return 1;
+        if (build_table(p, d, v, seg, rows_per_item, s)) return 1;
     }
     return 0;
 }
@@ -1937,7 +1954,9 @@ const Plan::ExtTable *ext_table(Plan &p, const Dom &d, int gen, int es, int en, 
         if (t.gen == gen && t.s == es && t.n == en) return &t;
     const int rf = d.ny_start - d.bnd_y1 - es, rl = d.ny_end - d.bnd_y1 + en;
     if (es < 0 || en < 0 || rf < 2 || rl + 2 > d.nya() - 1) return nullptr;
-    const std::vector<int4> items = partition(p, d, p.nsm * p.occ[gen], 0, rf, rl);
+    std::vector<Segment> seg = segments(p, d, rf, rl);
+    (void)cut_segments(p, seg, p.nsm * p.occ[gen], 0);
+    const std::vector<int4> items = work_items(p, d, seg, rf);
     Plan::ExtTable t{gen, es, en, (int)items.size(), nullptr};
     if (cudaMalloc(&t.items, items.size() * sizeof(int4)) != cudaSuccess) return nullptr;
     p.ext.push_back(t);   // owned by the plan from here on (freed by release)

@@ -108,7 +108,7 @@ struct Plan {
     int occ[5] = {0, 0, 0, 0, 0};   // resident CTAs per SM, per item table
     int occ_short[2] = {0, 0};      // the same with the short ring (plain FP64 substep)
     std::vector<uint8_t> ocean;     // per strip and interior row: any written column is ocean
-    int rows_per_item[2] = {0, 0};  // 0: cut by cost (partition); else about that many rows per item
+    int rows_per_item[2] = {0, 0};  // 0: cut by cost (cut_segments); else about that many rows per item
     int min_rows = 2;               // no work item is cut shorter (an ensemble member: 16)
     // plain-substep items over rows extended into the halo (a row strip
     // that advances several substeps per exchange): per variant and number
@@ -218,7 +218,7 @@ int prepare_steps_f32(Plan &p, const Dom &d, const Consts &c, double *state[6], 
 int launch_steps_f32(Plan &p, const Dom &d, const Consts &c, double dt, int nsteps, const double *rs_dev,
                      const int *rs_base, const double *rs_host, double *state[6], cudaStream_t s);
 int finish_steps_f32(Plan &p, const Dom &d, double *state[6], cudaStream_t s);
-// re-cut the work items: rows_per_item = 0 for chunks of equal cost (partition)
+// re-cut the work items: rows_per_item = 0 for chunks of equal cost (cut_segments)
 int repartition(Plan &p, const Dom &d, int rows_per_item, cudaStream_t s);
 // Persistent ensemble launch: one cooperative launch of one wave of CTAs
 // advances every member by `group` plain substeps (prepared by
