@@ -1380,24 +1380,27 @@ int upload_items(Plan &p, int v, const std::vector<int4> &items, int slots, int 
     return 0;
 }
 
-// Table v, cut for the resident CTAs of the ring its launches take: the short
-// one for the plain FP64 substep of a basin alone whose items make
-// SHORT_WAVES waves at most (us per substep with 5 and 4 slots: 4 waves,
-// 1700^2 73.7, 73.7 and 1800 x 1300 general 85.9, 85.0; 5 waves, 2048 x 1536
-// general 112, 114; 6 waves, 2048^2 102.9, 105.3).
+// Cuts table v's segments for the resident CTAs (slots) of the ring that its
+// launches take, and returns that ring: the short one for the plain FP64
+// substep of a basin alone whose items make SHORT_WAVES waves at most (us per
+// substep with 5 and 4 slots: 4 waves, 1700^2 73.7, 73.7 and 1800 x 1300
+// general 85.9, 85.0; 5 waves, 2048 x 1536 general 112, 114; 6 waves, 2048^2
+// 102.9, 105.3).
+int cut_for_ring(const Plan &p, int v, std::vector<Segment> &seg, int rows_per_item, int &slots)
+{
+    if (v <= 1 && p.min_rows <= 2) {
+        slots = p.nsm * p.occ_short[v];
+        if (cut_segments(p, seg, slots, rows_per_item) <= (long long)SHORT_WAVES * slots) return SHORT_RING;
+    }
+    slots = p.nsm * p.occ[v];
+    (void)cut_segments(p, seg, slots, rows_per_item);
+    return RING;
+}
+
 int build_table(Plan &p, const Dom &d, int v, std::vector<Segment> &seg, int rows_per_item, cudaStream_t s)
 {
-    int ring = RING, slots = p.nsm * p.occ[v];
-    if (v <= 1 && p.min_rows <= 2) {
-        ring = SHORT_RING;
-        slots = p.nsm * p.occ_short[v];
-    }
-    const long long n = cut_segments(p, seg, slots, rows_per_item);
-    if (ring == SHORT_RING && n > (long long)SHORT_WAVES * slots) {
-        ring = RING;
-        slots = p.nsm * p.occ[v];
-        (void)cut_segments(p, seg, slots, rows_per_item);
-    }
+    int slots = 0;
+    const int ring = cut_for_ring(p, v, seg, rows_per_item, slots);
     return upload_items(p, v, work_items(p, d, seg, d.ny_start - d.bnd_y1), slots, ring, s);
 }
 
@@ -1955,9 +1958,10 @@ const Plan::ExtTable *ext_table(Plan &p, const Dom &d, int gen, int es, int en, 
     const int rf = d.ny_start - d.bnd_y1 - es, rl = d.ny_end - d.bnd_y1 + en;
     if (es < 0 || en < 0 || rf < 2 || rl + 2 > d.nya() - 1) return nullptr;
     std::vector<Segment> seg = segments(p, d, rf, rl);
-    (void)cut_segments(p, seg, p.nsm * p.occ[gen], 0);
+    int slots = 0;
+    const int ring = cut_for_ring(p, gen, seg, 0, slots);
     const std::vector<int4> items = work_items(p, d, seg, rf);
-    Plan::ExtTable t{gen, es, en, (int)items.size(), nullptr};
+    Plan::ExtTable t{gen, es, en, (int)items.size(), ring, nullptr};
     if (cudaMalloc(&t.items, items.size() * sizeof(int4)) != cudaSuccess) return nullptr;
     p.ext.push_back(t);   // owned by the plan from here on (freed by release)
     if (cudaMemcpyAsync(t.items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, s) !=
@@ -1986,8 +1990,8 @@ int launch_step_ext(Plan &p, const Dom &d, const Consts &c, double dt, int ext_s
     if (set_io(p, q, state, p.buf[0])) return 1;
     q.items = t->items;
     p.last_variant = gen;
-    if (gen) launch_plain<true>(p.ring[1], t->nitems, q, s);
-    else launch_plain<false>(p.ring[0], t->nitems, q, s);
+    if (gen) launch_plain<true>(t->ring, t->nitems, q, s);
+    else launch_plain<false>(t->ring, t->nitems, q, s);
     if (cudaGetLastError() != cudaSuccess) return 1;
     for (int k = 0; k < 6; k++) std::swap(state[k], p.buf[0][k]);
     return 0;

@@ -114,7 +114,7 @@ struct Plan {
     // that advances several substeps per exchange): per variant and number
     // of rows computed south / north of the interior, built on first use
     struct ExtTable {
-        int gen, s, n, nitems;
+        int gen, s, n, nitems, ring;
         int4 *items;
     };
     std::vector<ExtTable> ext;
