@@ -427,6 +427,11 @@ int inmsom_gpu_path(inmsom_ctx *ctx, int *path, const char **reason);
  * calls compute normally. */
 int inmsom_test_hold_copy(inmsom_ctx *ctx, int item, int ring_row, unsigned wait_polls);
 
+/* Test hook: how many work items the fused path's table `table` holds (0, 1:
+ * plain substep, uniform and general variant; 2, 3: with time means; 4: FP32
+ * velocities) and the rows of the longest. */
+int inmsom_test_items(inmsom_ctx *ctx, int table, int *count, int *longest);
+
 /* Test hook: the context's device buffers for packed host copies take at
  * most `bytes` each from now on (as if the device had no more memory for
  * them); negative: the built-in 64 MB. */
@@ -609,7 +614,7 @@ int inmsom_read_checkpoint(inmsom_ctx *ctx, const char *path, double *ubrtr_e, d
  * every member's RHS at each substep.  group must be even (it keeps each
  * member's state in its set, so the graph can be replayed).  *ms receives
  * the device time of the run.  Creation re-cuts each member's work items
- * to 16 rows at least (a context alone cuts down to 1 or 2, which spreads a
+ * to about 16 rows or more (a context alone cuts down to 1 or 2, which spreads a
  * small basin over more SMs; in an ensemble the other members fill them),
  * and the members keep that cut after the ensemble is destroyed. */
 typedef struct inmsom_ens inmsom_ens;

@@ -34,7 +34,7 @@ EXPORTS = (
     "inmsom_write_checkpoint", "inmsom_read_checkpoint", "inmsom_tracer_tran_diff", "inmsom_ctl_file_read",
     "inmsom_pwdstd", "inmsom_prdstd", "inmsom_ocpwrite", "inmsom_ocpread",
     "inmsom_compare_grids", "inmsom_stress_components", "inmsom_smagorinsky_coeff",
-    "inmsom_test_hold_copy", "inmsom_test_stage_limit", "inmsom_test_stage_allocs", "inmsom_step_launch_rows", "inmsom_gpu_halo", "inmsom_ens_persistent",
+    "inmsom_test_hold_copy", "inmsom_test_items", "inmsom_test_stage_limit", "inmsom_test_stage_allocs", "inmsom_step_launch_rows", "inmsom_gpu_halo", "inmsom_ens_persistent",
 )
 
 # include/inmsom_gpu.h: INMSOM_MLP_*
@@ -121,6 +121,7 @@ def load() -> ctypes.CDLL:
     lib.inmsom_load_state.argtypes = [VP] + [DP] * 12
     lib.inmsom_gpu_path.argtypes = [VP, ctypes.POINTER(i), ctypes.POINTER(ctypes.c_char_p)]
     lib.inmsom_test_hold_copy.argtypes = [VP, i, i, ctypes.c_uint]
+    lib.inmsom_test_items.argtypes = [VP, i, ctypes.POINTER(i), ctypes.POINTER(i)]
     lib.inmsom_test_stage_limit.argtypes = [VP, ctypes.c_longlong]
     lib.inmsom_test_stage_allocs.argtypes = [VP, ctypes.POINTER(i)]
     lib.inmsom_gpu_finalize.argtypes = [VP]

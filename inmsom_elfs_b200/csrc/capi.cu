@@ -414,6 +414,14 @@ int inmsom_test_hold_copy(inmsom_ctx *c, int item, int ring_row, unsigned wait_p
     return INMSOM_OK;
 }
 
+int inmsom_test_items(inmsom_ctx *c, int table, int *count, int *longest)
+{
+    if (!c || !count || !longest || table < 0 || table > 4) return set_err(INMSOM_EARG, "inmsom_test_items: bad argument");
+    *count = c->plan.nitems[table];
+    *longest = c->plan.longest[table];
+    return INMSOM_OK;
+}
+
 int inmsom_test_stage_limit(inmsom_ctx *c, long long bytes)
 {
     if (!c) return set_err(INMSOM_EARG, "NULL context");
@@ -1152,7 +1160,7 @@ int inmsom_gpu_sync_from_host(inmsom_ctx *c, unsigned what)
 
 // ===========================================================================
 // Ensemble of contexts advanced by one CUDA graph per group of substeps.
-constexpr int ENS_MIN_ROWS = 16;   // shortest work item of an ensemble member
+constexpr int ENS_MIN_ROWS = 16;   // rows of an ensemble member's work item, about, or more
 
 struct inmsom_ens {
     std::vector<inmsom_ctx *> m;
@@ -1282,7 +1290,7 @@ int inmsom_ens_create(inmsom_ens **out, inmsom_ctx *const *members, int n, int g
     e->join.assign(n, nullptr);
     for (int i = 0; i < n && ce == cudaSuccess; i++) ce = cudaEventCreateWithFlags(&e->join[i], cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaMalloc(&e->d_base, sizeof(int));
-    // members share the device: items of 16 rows at least (a basin alone
+    // members share the device: items of about 16 rows or more (a basin alone
     // cuts down to 1 or 2 to spread a small basin over more SMs)
     for (int i = 0; i < n && ce == cudaSuccess; i++) {
         inmsom_ctx *c = members[i];

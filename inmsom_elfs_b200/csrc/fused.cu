@@ -1246,12 +1246,17 @@ std::vector<uint8_t> ocean_rows(const Plan &p, const Dom &d, const float *lu)
 // FP32 velocities: 373, 335, 327, 322 us).  A land row inside a segment
 // skips the momentum stages and costs about LAND_COST of an ocean row.
 //
-// No chunk is cut shorter than p.min_rows rows (16 for an ensemble member,
-// whose neighbours fill the SMs).  A basin alone goes down to 2 rows, and to
-// 1 where that is at most 3/4 of a wave: such a basin is bound by the latency
-// of an item's chain of rows (us per substep with 4, 2 and 1 rows: 256^2
-// basin, 2286 rows in all: 8.1, 5.4, 6.1; 300 x 200 with land, 1500 rows:
-// 8.5, 6.7, 5.9; 64^2: 8.0, 4.7, 3.8).
+// A segment makes no more chunks than its rows / p.min_rows: chunks of 2 rows
+// or more on average for a basin alone, and of 1 where that is at most 3/4 of
+// a wave (such a basin is bound by the latency of an item's chain of rows; us
+// per substep with 4, 2 and 1 rows: 256^2 basin, 2286 rows in all: 8.1, 5.4,
+// 6.1; 300 x 200 with land, 1500 rows: 8.5, 6.7, 5.9; 64^2: 8.0, 4.7, 3.8).
+// For an ensemble member, whose neighbours fill the SMs, it is 16, to the
+// nearest: rounded down, segments of up to 31 rows stayed whole, and a few
+// members waited for their chains (us per substep of regional basins rounded
+// down and to the nearest, graph form then persistent: 2 members 24.4, 18.9
+// and 53.1, 44.5; 5 members 24.9, 20.9 and 55.8, 44.7; 10 members 56.6, 55.9
+// and 70.4, 69.0; 64 members 376, 371 and 430, 432).
 constexpr int GAP_ROWS = 8;     // longest run of land rows inside an item
 constexpr double WARM = 2.5;    // an item's warm-up iterations, in ocean rows
 constexpr int WAVE_ROWS = 10, MAX_WAVES = 8;
@@ -1294,7 +1299,8 @@ long long cut_segments(const Plan &p, std::vector<Segment> &seg, int slots, int 
     long long rows = 0, all = 0;
     for (const Segment &g : seg) rows += g.r1 - g.r0 + 1;
     const int min_rows = p.min_rows <= 2 && rows <= slots * 3LL / 4 ? 1 : std::max(1, p.min_rows);
-    auto most = [&](const Segment &g) { return std::max(1, (g.r1 - g.r0 + 1) / min_rows); };
+    const int round = p.min_rows > 2 ? min_rows / 2 : 0;
+    auto most = [&](const Segment &g) { return std::max(1, (g.r1 - g.r0 + 1 + round) / min_rows); };
     if (rows_per_item > 0) {
         for (Segment &g : seg) {
             g.n = std::min(most(g), std::max(1, (g.r1 - g.r0 + 1 + rows_per_item / 2) / rows_per_item));
@@ -1374,7 +1380,11 @@ int upload_items(Plan &p, int v, const std::vector<int4> &items, int slots, int 
     // -> 51.1, the drop-in call's 100 substeps 7.71 -> 7.49 ms; with one wave
     // or past L2 it lost 1-6 %: 512^2 10.0 -> 10.7, 4096^2 FP32 300 -> 302 us).
     double rows = 0.0;
-    for (const int4 &it : items) rows += it.z - it.y;
+    p.longest[v] = 0;
+    for (const int4 &it : items) {
+        rows += it.z - it.y;
+        p.longest[v] = std::max(p.longest[v], it.z - it.y);
+    }
     const double cell = v == TABLE_F32 ? 80.0 : (v == 2 || v == 3 ? 184.0 : 120.0);
     p.turn[v] = p.nitems[v] > slots && rows * p.outw * cell * slots / p.nitems[v] <= L2_BYTES;
     return 0;

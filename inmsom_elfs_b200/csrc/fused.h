@@ -92,6 +92,7 @@ struct Plan {
     int nitems[5] = {0, 0, 0, 0, 0};
     int4 *items[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // {g0, first row, end row, strip} per item
     int ring[5] = {5, 5, 5, 5, 5};  // ring slots its launches take
+    int longest[5] = {};      // rows of a table's longest item
     bool turn[5] = {};        // alternate substeps take a table's items from its end
     bool uni = false;         // metrics all equal one spacing d (square uniform grid)
     double d = 0.0;           // that spacing
@@ -109,7 +110,7 @@ struct Plan {
     int occ_short[2] = {0, 0};      // the same with the short ring (plain FP64 substep)
     std::vector<uint8_t> ocean;     // per strip and interior row: any written column is ocean
     int rows_per_item[2] = {0, 0};  // 0: cut by cost (cut_segments); else about that many rows per item
-    int min_rows = 2;               // no work item is cut shorter (an ensemble member: 16)
+    int min_rows = 2;               // a segment's items have as many rows on average, or more (an ensemble member: about 16)
     // plain-substep items over rows extended into the halo (a row strip
     // that advances several substeps per exchange): per variant and number
     // of rows computed south / north of the interior, built on first use
