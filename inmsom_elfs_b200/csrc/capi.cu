@@ -297,7 +297,6 @@ int inmsom_gpu_finalize(inmsom_ctx *c)
     cudaFree(c->trc_lev);
     transfer::release(c->stage);
     transfer::release(c->stage_up);
-    transfer::release(c->stage_dn);
     for (auto &e : c->bev)
         if (e) cudaEventDestroy(e);
     if (c->s_up) cudaStreamDestroy(c->s_up);
@@ -425,7 +424,7 @@ int inmsom_test_items(inmsom_ctx *c, int table, int *count, int *longest)
 int inmsom_test_stage_limit(inmsom_ctx *c, long long bytes)
 {
     if (!c) return set_err(INMSOM_EARG, "NULL context");
-    for (transfer::Stage *st : {&c->stage, &c->stage_up, &c->stage_dn}) {
+    for (transfer::Stage *st : {&c->stage, &c->stage_up}) {
         transfer::release(*st);
         st->limit = bytes < 0 ? transfer::STAGE_BYTES : (size_t)bytes;
     }
@@ -435,7 +434,7 @@ int inmsom_test_stage_limit(inmsom_ctx *c, long long bytes)
 int inmsom_test_stage_allocs(inmsom_ctx *c, int *count)
 {
     if (!c || !count) return set_err(INMSOM_EARG, "NULL argument");
-    *count = c->stage.allocs + c->stage_up.allocs + c->stage_dn.allocs;
+    *count = c->stage.allocs + c->stage_up.allocs;
     return INMSOM_OK;
 }
 

@@ -74,27 +74,23 @@ int pipelined(inmsom_ctx *c, int nb, const std::vector<Field> &pre, const double
     const int iy0 = d.ny_start - d.bnd_y1, iy1 = d.ny_end - d.bnd_y1;
     auto failed = [] { return set_err(INMSOM_ECUDA, "launch failed: %s", cudaGetErrorString(cudaGetLastError())); };
     auto up = [&](const std::vector<Field> &f, int r0, int r1) {
-        return transfer::rows(c->stage_up, d, f.data(), (int)f.size(), r0, r1, true, c->s_up);
+        return transfer::upload(c->stage_up, d, f.data(), (int)f.size(), r0, r1, c->s_up);
     };
     auto down = [&](int r0, int r1) {
-        return transfer::rows(c->stage_dn, d, out.data(), (int)out.size(), r0, r1, false, c->s_dn);
+        return transfer::download(d, out.data(), (int)out.size(), r0, r1, c->s_dn);
     };
     // band b: interior rows first(b) .. first(b+1)-1, uploaded up to (not
     // including) array row up_end(b)
     auto first = [&](int b) { return d.ny_start + (int)((long long)nyi * b / nb); };
     auto up_end = [&](int b) { return b == nb - 1 ? nya : first(b + 1) + 1 - d.bnd_y1; };
-    // both stages at the largest band's size before the first copy: to grow
-    // one later would wait for the copies under way
-    int most_up = 0, most_dn = std::max(iy0, nya - 1 - iy1);
-    for (int b = 0; b < nb; b++) {
-        most_up = std::max(most_up, up_end(b) - (b ? up_end(b - 1) : 0));
-        most_dn = std::max(most_dn, first(b + 1) - first(b));
-    }
+    // the stage at the largest band's size before the first copy: to grow it
+    // later would wait for the copies under way
+    int most = 0;
+    for (int b = 0; b < nb; b++) most = std::max(most, up_end(b) - (b ? up_end(b - 1) : 0));
     auto bytes = [&](const std::vector<Field> &f, int nrows) {
         return transfer::packed_bytes(d, f.data(), (int)f.size(), nrows);
     };
-    CK(transfer::reserve(c->stage_up, std::max(bytes(pre, nya), bytes(in, most_up))));
-    CK(transfer::reserve(c->stage_dn, bytes(out, most_dn)));
+    CK(transfer::reserve(c->stage_up, std::max(bytes(pre, nya), bytes(in, most))));
     c->ph_valid = false;
     c->ph_direct = false;
     CK(cudaEventRecord(c->ph[0], c->stream));

@@ -87,7 +87,7 @@ struct inmsom_ctx {
     cudaEvent_t bev[4 * 8 + 4] = {};
     float ph_ms[3] = {};
     bool ph_direct = false;
-    transfer::Stage stage, stage_up, stage_dn;   // packed rows on their way: on stream, s_up, s_dn
+    transfer::Stage stage, stage_up;   // packed rows on their way: on stream, on s_up
     // inmsom_tracer_tran_diff: fields of trc_nz levels in one block and dz, hzt
     double *trc = nullptr, *trc_lev = nullptr;
     int trc_nz = 0;
@@ -158,8 +158,7 @@ int dalloc(inmsom_ctx *c, T **p, size_t elem)
 }
 
 // Whole fields between host arrays and the device, collected by add and
-// enqueued together on the context's stream (one kernel packs or unpacks
-// short rows of all of them)
+// enqueued together on the context's stream
 class Copies {
   public:
     explicit Copies(inmsom_ctx *ctx) : c(ctx) {}
@@ -170,23 +169,26 @@ class Copies {
         f.push_back({(void *)dev, (void *)host, nlev, (int)sizeof(T)});
         return INMSOM_OK;
     }
-    int up() { return go(true); }
-    int down() { return go(false); }
+    int up()
+    {
+        // one allocation for the life of the context: as many fields as an
+        // upload packs at once
+        const std::vector<transfer::Field> most(transfer::MAX_PIECES, {nullptr, nullptr, 1, (int)sizeof(double)});
+        CK(transfer::reserve(c->stage, transfer::packed_bytes(c->dom, most.data(), (int)most.size(), c->dom.nya())));
+        CK(transfer::upload(c->stage, c->dom, f.data(), (int)f.size(), 0, c->dom.nya() - 1, c->stream));
+        f.clear();
+        return INMSOM_OK;
+    }
+    int down()
+    {
+        CK(transfer::download(c->dom, f.data(), (int)f.size(), 0, c->dom.nya() - 1, c->stream));
+        f.clear();
+        return INMSOM_OK;
+    }
 
   private:
     inmsom_ctx *c;
     std::vector<transfer::Field> f;
-    int go(bool to_device)
-    {
-        // one allocation for the life of the context: the largest 2-D call
-        // moves the state, the scratch, the forcing and the depths
-        constexpr size_t most = NSTATE + NSCR + NFORC + NDEPTH;
-        const transfer::Field one{nullptr, nullptr, 1, (int)sizeof(double)};
-        CK(transfer::reserve(c->stage, most * transfer::packed_bytes(c->dom, &one, 1, c->dom.nya())));
-        CK(transfer::rows(c->stage, c->dom, f.data(), (int)f.size(), 0, c->dom.nya() - 1, to_device, c->stream));
-        f.clear();
-        return INMSOM_OK;
-    }
 };
 
 // one field
