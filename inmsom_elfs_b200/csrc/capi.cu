@@ -924,13 +924,15 @@ int inmsom_ssh_internal(inmsom_ctx *c, double tau, double *ssh_i, double *sshp_i
     CKR(ensure_grid(c));
     CKR(alloc_set(c, c->intl, NINT));
     double **I = c->intl;
-    CKR(h2d(c, I[I_SSH], (const double *)ssh_i));
-    CKR(h2d(c, I[I_SSHP], (const double *)sshp_i));
-    CKR(h2d(c, I[I_U], u));
-    CKR(h2d(c, I[I_V], v));
-    CKR(h2d(c, I[I_WFLUX], wflux));
     double *hi[4] = {hhqn, hhun, hhvn, hhhn};
-    for (int k = 0; k < 4; k++) CKR(h2d(c, I[I_HQN + k], (const double *)hi[k]));
+    Copies q(c);
+    CKR(q.add(I[I_SSH], (const double *)ssh_i));
+    CKR(q.add(I[I_SSHP], (const double *)sshp_i));
+    CKR(q.add(I[I_U], u));
+    CKR(q.add(I[I_V], v));
+    CKR(q.add(I[I_WFLUX], wflux));
+    for (int k = 0; k < 4; k++) CKR(q.add(I[I_HQN + k], (const double *)hi[k]));
+    CKR(q.up());
     const Dom &d = c->dom;
     const GridDev g = c->gdev();
     general::fill(d, I[I_NEW], 0.0, c->stream);  // vel_ssh.f90:704-705
@@ -939,9 +941,10 @@ int inmsom_ssh_internal(inmsom_ctx *c, double tau, double *ssh_i, double *sshp_i
     if (c->c.ffs > 0)
         general::hh_update(d, g, I[I_HQN], I[I_HUN], I[I_HVN], I[I_HHN], I[I_NEW], c->stream);
     general::asselin_ssh(d, g, c->c, I[I_SSH], I[I_SSHP], I[I_NEW], c->stream);
-    CKR(d2h(c, ssh_i, I[I_SSH]));
-    CKR(d2h(c, sshp_i, I[I_SSHP]));
-    for (int k = 0; k < 4; k++) CKR(d2h(c, hi[k], I[I_HQN + k]));
+    CKR(q.add(I[I_SSH], (const double *)ssh_i));
+    CKR(q.add(I[I_SSHP], (const double *)sshp_i));
+    for (int k = 0; k < 4; k++) CKR(q.add(I[I_HQN + k], (const double *)hi[k]));
+    CKR(q.down());
     return sync_stream(c);
 }
 
@@ -992,14 +995,17 @@ int inmsom_wind_forcing(inmsom_ctx *c, const double *taux, const double *tauy, d
     CKR(ensure_grid(c));
     for (int k = 0; k < 4; k++)
         if (!c->tmp[k]) CKR(dalloc(c, &c->tmp[k], sizeof(double)));
-    CKR(h2d(c, c->tmp[0], taux));
-    CKR(h2d(c, c->tmp[1], tauy));
-    CKR(h2d(c, c->tmp[2], (const double *)RHSx2d));
-    CKR(h2d(c, c->tmp[3], (const double *)RHSy2d));
+    Copies q(c);
+    CKR(q.add(c->tmp[0], taux));
+    CKR(q.add(c->tmp[1], tauy));
+    CKR(q.add(c->tmp[2], (const double *)RHSx2d));
+    CKR(q.add(c->tmp[3], (const double *)RHSy2d));
+    CKR(q.up());
     general::wind_forcing(c->dom, c->gdev(), c->c, c->tmp[0], c->tmp[1], c->tmp[2], c->tmp[3],
                           c->stream);
-    CKR(d2h(c, RHSx2d, c->tmp[2]));
-    CKR(d2h(c, RHSy2d, c->tmp[3]));
+    CKR(q.add(c->tmp[2], (const double *)RHSx2d));
+    CKR(q.add(c->tmp[3], (const double *)RHSy2d));
+    CKR(q.down());
     return sync_stream(c);
 }
 
@@ -1016,32 +1022,36 @@ int inmsom_rhs2d(inmsom_ctx *c, double *RHSx2d, double *RHSy2d, const double *RH
     double **r = c->r2d, *zero = c->r2d[6];
     // an input on the device, or the zero field for a NULL argument (a
     // missing term adds or subtracts 0, as in the reference with the term zero)
-    auto in = [&](double *dev, const double *host, int *rc) -> const double * {
+    Copies q(c);
+    int rc = INMSOM_OK;
+    auto in = [&](double *dev, const double *host) -> const double * {
         if (!host) return zero;
-        *rc = h2d(c, dev, host);
+        if (rc == INMSOM_OK) rc = q.add(dev, host);
         return dev;
     };
-    int rc = INMSOM_OK;
-    CKR(h2d(c, r[0], (const double *)RHSx2d));
-    CKR(h2d(c, r[1], (const double *)RHSy2d));
+    CKR(q.add(r[0], (const double *)RHSx2d));
+    CKR(q.add(r[1], (const double *)RHSy2d));
     const GridDev g = c->gdev();
     const double *pairs[3][2] = {{RHSx2d_diff_disp, RHSy2d_diff_disp}, {RHSx2d_tran, RHSy2d_tran},
                                  {RHSx2d_tran_disp, RHSy2d_tran_disp}};
     const int term_of[3] = {0, 1, 0};
     for (int t = 0; t < 3; t++) {
-        const double *ax = in(r[2], pairs[t][0], &rc), *ay = in(r[3], pairs[t][1], &rc);
+        const double *ax = in(r[2], pairs[t][0]), *ay = in(r[3], pairs[t][1]);
         CKR(rc);
+        CKR(q.up());
         general::rhs2d_term(c->dom, g, c->c, term_of[t], r[0], r[1], ax, ay, nullptr, nullptr, c->stream);
     }
     {
-        const double *ax = in(r[2], surf_stress_x, &rc), *bx = in(r[3], bot_stress_x, &rc);
-        const double *ay = in(r[4], surf_stress_y, &rc), *by = in(r[5], bot_stress_y, &rc);
+        const double *ax = in(r[2], surf_stress_x), *bx = in(r[3], bot_stress_x);
+        const double *ay = in(r[4], surf_stress_y), *by = in(r[5], bot_stress_y);
         CKR(rc);
+        CKR(q.up());
         general::rhs2d_term(c->dom, g, c->c, 2, r[0], r[1], ax, ay, bx, by, c->stream);
     }
     {
-        const double *a = in(r[2], slpr, &rc), *bx = in(r[3], hhu, &rc), *by = in(r[4], hhv, &rc);
+        const double *a = in(r[2], slpr), *bx = in(r[3], hhu), *by = in(r[4], hhv);
         CKR(rc);
+        CKR(q.up());
         general::rhs2d_term(c->dom, g, c->c, 3, r[0], r[1], a, a, bx, by, c->stream);
     }
     CK(cudaGetLastError());
@@ -1063,19 +1073,24 @@ int inmsom_velocity2d(inmsom_ctx *c, double *uu2d, double *vv2d, double *pgrx, d
         if (!p) return set_err(INMSOM_EARG, "inmsom_velocity2d: NULL argument");
     CKR(alloc_block(c, c->v2d, 9));
     double **v = c->v2d;
-    for (int k = 0; k < 4; k++) CKR(h2d(c, v[k], (const double *)out[k]));
-    for (int k = 0; k < 5; k++) CKR(h2d(c, v[4 + k], in[k]));
+    Copies q(c);
+    for (int k = 0; k < 4; k++) CKR(q.add(v[k], (const double *)out[k]));
+    for (int k = 0; k < 5; k++) CKR(q.add(v[4 + k], in[k]));
+    CKR(q.up());
     general::velocity2d(c->dom, c->gdev(), c->c, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7], v[8], c->stream);
     CK(cudaGetLastError());
-    for (int k = 0; k < 4; k++) CKR(d2h(c, out[k], v[k]));
+    for (int k = 0; k < 4; k++) CKR(q.add(v[k], (const double *)out[k]));
+    CKR(q.down());
     return sync_stream(c);
 }
 
 int inmsom_hh_init_external(inmsom_ctx *c, const double *ssh_e, const double *sshp_e)
 {
     CKR(ensure_grid(c));
-    CKR(h2d(c, c->state[S_SSH], ssh_e));
-    CKR(h2d(c, c->state[S_SSHP], sshp_e));
+    Copies q(c);
+    CKR(q.add(c->state[S_SSH], ssh_e));
+    CKR(q.add(c->state[S_SSHP], sshp_e));
+    CKR(q.up());
     fused::mark_state_changed(c->plan);
     depths_from_state(c);
     for (int k = 0; k < NDEPTH; k++)
@@ -1133,8 +1148,8 @@ int inmsom_gpu_sync_to_host(inmsom_ctx *c, unsigned what)
 int inmsom_gpu_sync_from_host(inmsom_ctx *c, unsigned what)
 {
     CKR(ensure_grid(c));
+    Copies in(c);
     if (what & INMSOM_SYNC_STATE) {
-        Copies in(c);
         for (int k = 0; k < NSTATE; k++) CKR(in.add(c->state[k], (const double *)c->h_state[k]));
         CKR(in.up());
         c->state_on_device = true;
@@ -1143,11 +1158,13 @@ int inmsom_gpu_sync_from_host(inmsom_ctx *c, unsigned what)
     }
     if (what & INMSOM_SYNC_DEPTHS) {
         for (int k = 0; k < NDEPTH; k++)
-            if (c->h_depth[k]) CKR(h2d(c, c->depth[k], (const double *)c->h_depth[k]));
+            if (c->h_depth[k]) CKR(in.add(c->depth[k], (const double *)c->h_depth[k]));
+        CKR(in.up());
         c->depths_current = true;
     }
     if (what & INMSOM_SYNC_SCRATCH) {
-        for (int k = 0; k < NSCR; k++) CKR(h2d(c, c->scr[k], (const double *)c->h_scr[k]));
+        for (int k = 0; k < NSCR; k++) CKR(in.add(c->scr[k], (const double *)c->h_scr[k]));
+        CKR(in.up());
         c->scratch_on_device = true;
     }
     if (what & INMSOM_SYNC_COEFFS)

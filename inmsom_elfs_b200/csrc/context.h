@@ -173,8 +173,9 @@ class Copies {
     {
         // one allocation for the life of the context: as many fields as an
         // upload packs at once
-        const std::vector<transfer::Field> most(transfer::MAX_PIECES, {nullptr, nullptr, 1, (int)sizeof(double)});
-        CK(transfer::reserve(c->stage, transfer::packed_bytes(c->dom, most.data(), (int)most.size(), c->dom.nya())));
+        transfer::Field most[transfer::MAX_PIECES];
+        for (auto &m : most) m = {nullptr, nullptr, 1, (int)sizeof(double)};
+        CK(transfer::reserve(c->stage, transfer::packed_bytes(c->dom, most, transfer::MAX_PIECES, c->dom.nya())));
         CK(transfer::upload(c->stage, c->dom, f.data(), (int)f.size(), 0, c->dom.nya() - 1, c->stream));
         f.clear();
         return INMSOM_OK;
