@@ -198,9 +198,14 @@ constexpr size_t ring_bytes(int slots = RING)
 // slower; reading the forcing from global memory instead of the ring exposes
 // the load latency: 5 % slower.)
 template <bool GEN, int MODE, bool F32 = false>
+constexpr int ctas_by_smem(int slots = RING)
+{
+    return (int)(233472 / (ring_bytes<GEN, MODE, F32>(slots) + 1024));
+}
+template <bool GEN, int MODE, bool F32 = false>
 constexpr int min_ctas()
 {
-    constexpr int by_smem = (int)(233472 / (ring_bytes<GEN, MODE, F32>(MODE == 3 && !F32 ? SHORT_RING : RING) + 1024));
+    constexpr int by_smem = ctas_by_smem<GEN, MODE, F32>(MODE == 3 && !F32 ? SHORT_RING : RING);
     constexpr int want = GEN ? 12 : (MODE % 3 ? 12 : (F32 ? 20 : 16));
     return by_smem < want ? by_smem : want;
 }
@@ -862,14 +867,14 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *a)
     return v;
 }
 
-// resident CTAs per SM the kernel is cut for: the general variant's where
-// some member takes it, else 12 (on 64 regional basins 16 CTAs, at 128
-// registers with a few bytes spilled, ran 8 % slower, 11 CTAs 10 % slower,
-// and 8, 10 and 12 alike)
+// resident CTAs per SM the kernel is cut for: where some member takes the
+// general variant what its ring of five slots leaves room for (11), else 12
+// (on 64 regional basins 16 CTAs, at 128 registers with a few bytes spilled,
+// ran 8 % slower, 11 CTAs 10 % slower, and 8, 10 and 12 alike)
 template <bool ANYGEN>
 constexpr int ens_ctas()
 {
-    return ANYGEN ? min_ctas<true, 3>() : 12;
+    return ANYGEN ? ctas_by_smem<true, 3>() : 12;
 }
 constexpr unsigned ENS_WAIT_POLLS = 1u << 16;
 
