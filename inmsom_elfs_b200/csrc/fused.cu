@@ -1358,7 +1358,6 @@ std::vector<int4> work_items(const Plan &p, const Dom &d, const std::vector<Segm
     return items;
 }
 
-constexpr double L2_BYTES = 126e6;
 constexpr int SHORT_WAVES = 4;
 
 // Replaces table v.  On failure the plan keeps its previous table (a
@@ -1391,7 +1390,7 @@ int upload_items(Plan &p, int v, const std::vector<int4> &items, int slots, int 
         p.longest[v] = std::max(p.longest[v], it.z - it.y);
     }
     const double cell = v == TABLE_F32 ? 80.0 : (v == 2 || v == 3 ? 184.0 : 120.0);
-    p.turn[v] = p.nitems[v] > slots && rows * p.outw * cell * slots / p.nitems[v] <= L2_BYTES;
+    p.turn[v] = p.nitems[v] > slots && rows * p.outw * cell * slots / p.nitems[v] <= p.l2;
     return 0;
 }
 
@@ -1709,6 +1708,7 @@ int setup(Plan &p, const Dom &d, const Consts &c, const float *const masks[7], c
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     p.nsm = nsm;
+    cudaDeviceGetAttribute(&p.l2, cudaDevAttrL2CacheSize, dev);
     // one item table per variant for the plain substep and one for the
     // time-mean substeps, cut for the kernel's resident CTAs
     auto occupancy = [](int &n, const void *kernel, size_t smem) {

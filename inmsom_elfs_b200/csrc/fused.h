@@ -141,7 +141,7 @@ struct Plan {
     double *d_uniform = nullptr;    // per-block min/max of mu, rdis, wflux
     unsigned *d_flags = nullptr;    // [0] status bits (guard / timeout)
     const float *lu = nullptr;      // borrowed
-    int nsm = 148;
+    int nsm = 148, l2 = 0;          // SMs, bytes of L2
     bool vort_zero = false;
     bool buffers_synced = false;    // buf[][] hold the state's land/halo values
     unsigned last_flags = 0;        // status bits of the last run
