@@ -305,7 +305,8 @@ __device__ __forceinline__ R rcount(int n)
 // correctly rounded single-precision reciprocal, with its conversions and
 // its slow-path branch, a substep took 62.5 instead of 59.0 us on 2048 x
 // 1536, 5.15 instead of 4.46 on 256^2, 16.6 instead of 14.2 on a 701 x 487
-// spherical basin; the same results bit for bit.)
+// spherical basin.  On 5.4e8 random values from 1/16 to 65536 both give the
+// correctly rounded reciprocal every time.)  0 and infinity give NaN.
 __device__ __forceinline__ double rcp_nr(double x)
 {
     double r;
@@ -315,9 +316,11 @@ __device__ __forceinline__ double rcp_nr(double x)
     e = fma(-x, r, 1.0);
     return fma(r, e, r);
 }
-// the FP32 reciprocal: one Newton step from the hardware's approximation
-// (the correctly rounded function has a slow-path branch: 51.0 instead of
-// 45.3 us per substep on 2048 x 1536)
+// the FP32 reciprocal: one Newton step from the hardware's approximation.
+// Compared with the correctly rounded function on every significand with
+// every exponent from 2^-60 to 2^60: never different.  (That function has a
+// slow-path branch: 51.0 instead of 45.3 us per substep on 2048 x 1536.)  0
+// and infinity give NaN.
 __device__ __forceinline__ float rcp_nr(float x)
 {
     float r;
