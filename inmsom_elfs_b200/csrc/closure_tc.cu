@@ -226,17 +226,12 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
     }
     // Launched with programmatic stream serialisation: what follows reads what
     // earlier kernels of the stream wrote (the weights, the batch).  The
-    // tensor memory is taken only now: the stream's last kernel may be
-    // another program's that takes tensor memory after it let this one in,
-    // and would wait for columns held by a CTA that waits for its end.
+    // tensor memory is taken after it too, while the first loads are under
+    // way: the stream's last kernel may be another program's that takes
+    // tensor memory after it let this one in, and would wait for columns held
+    // by a CTA that waits for its end.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     fetch(blockIdx.x);
-    if (w == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&s.tmem_base)),
-                     "r"(TM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
     // weights, 16 bytes (8 outputs of one input) at a time
     {
         constexpr int G = HID / 8, N1 = KIN * G, N2 = HID * G;   // pieces
@@ -250,6 +245,12 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM)
             if (i < N2) p2[h] = w16[(BOFF_W2 / 8) + i];
         }
         if (t < HID) p3 = w16[(BOFF_W3 / 8) + t];
+        if (w == 0) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&s.tmem_base)),
+                         "r"(TM_COLS)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int i = t + h * THREADS;
