@@ -26,8 +26,8 @@
 // fit), and DZ2, DZ1 go over A2, A1 in shared memory once those are used up
 // (86 KB).  A tile's dW1 is issued with the next tile's Z1 (X has two
 // buffers): five steps per tile, one barrier and one wait each.  Measured
-// (gradient, reduction and Adam): 23.7 us per training step at batch 65536,
-// 12.2 at 1024, against 42.0 and 22.6 with one CTA of sixteen warps, seven
+// (gradient, reduction and Adam): 24.4 us per training step at batch 65536,
+// 12.0 at 1024, against 42.0 and 22.6 with one CTA of sixteen warps, seven
 // steps per tile and the partial sums stored row by row.  The two CTAs leave
 // 128 registers per thread, of which the compiler spills 18 bytes.
 // The bias gradients come out of the same weight-gradient products: X, A1
